@@ -1829,6 +1829,12 @@ __global__ void __launch_bounds__(KR_THREADS, 2) k_cg1_cluster(KArgs<T> a) {
     }
 }
 
+}  // namespace pict
+
+#include "krylov_resident.cuh"
+
+namespace pict {
+
 __global__ void k_init_info(pict_solve_info_t* info, int n) {
     PICT_CELL_LOOP(i, n) {
         info[i].final_residual = 0.0;
@@ -1928,6 +1934,87 @@ static pict_status_t launch_cg1_cluster(KArgs<T>& a, int cl, cudaStream_t st) {
     return PICT_OK;
 }
 
+// ---- resident solves (krylov_resident.cuh)
+
+// Cells per thread a resident solve of this domain needs with clusters of 16 CTAs (the largest system decides;
+// every system of the domain then takes the resident path, so a batch and its members alone sum in the same order).
+static int resident_cpt(const pict_domain_t* dom) {
+    const long long per_cta = ((long long)dom->max_sim_cells + KC_MAX_CL - 1) / KC_MAX_CL;
+    return (int)((per_cta + RS_THREADS - 1) / RS_THREADS);
+}
+
+// Launch `kern` in clusters of 16 CTAs with `smem` bytes each, as many clusters as fit at once (at most one per
+// system).  PICT_ERR_UNSUPPORTED (nothing launched) where no such cluster fits on the device.
+template <typename T>
+static pict_status_t launch_resident(void (*kern)(KArgs<T>, bool), size_t smem, KArgs<T>& a, bool trans, cudaStream_t st) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        return PICT_ERR_UNSUPPORTED;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(RS_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = KC_MAX_CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(KC_MAX_CL);
+    int ncl = 0;
+    if (cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) != cudaSuccess || ncl < 1) {
+        cudaGetLastError();
+        return PICT_ERR_UNSUPPORTED;
+    }
+    if (ncl > a.dom.num_sims) ncl = a.dom.num_sims;
+    cfg.gridDim = dim3(ncl * KC_MAX_CL);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, trans);
+    if (e != cudaSuccess) {
+        char buf[256];
+        snprintf(buf, sizeof(buf), "resident solve launch (%d clusters): %s", ncl, cudaGetErrorString(e));
+        cudaGetLastError();
+        return set_error(PICT_ERR_CUDA, buf);
+    }
+    return PICT_OK;
+}
+
+template <typename T, int D, int CPT, bool ROWS_SMEM>
+static pict_status_t launch_cg1_resident_as(KArgs<T>& a, bool trans, cudaStream_t st) {
+    return launch_resident<T>(k_cg1_resident<T, D, CPT, ROWS_SMEM>, resident_smem<T, D, CPT, ROWS_SMEM>(1), a, trans, st);
+}
+
+// The stencil rows stay in registers while a thread's share fits 128 of them: up to 4 FP32 cells, 1 FP64 cell (2 in
+// 2D).  Beyond that they go to shared memory, up to 8 FP32 / 4 FP64 cells (65,536 / 32,768 cells a system).
+template <typename T, int D>
+static pict_status_t launch_cg1_resident(KArgs<T>& a, bool trans, cudaStream_t st) {
+    const int cpt = resident_cpt(&a.dom);
+    if (cpt <= 1) return launch_cg1_resident_as<T, D, 1, false>(a, trans, st);
+    if (cpt <= 2) return launch_cg1_resident_as<T, D, 2, sizeof(T) == 8 && D == 3>(a, trans, st);
+    if (cpt <= 4) return launch_cg1_resident_as<T, D, 4, sizeof(T) == 8>(a, trans, st);
+    if constexpr (sizeof(T) == 4)
+        if (cpt <= 8) return launch_cg1_resident_as<T, D, 8, true>(a, trans, st);
+    return PICT_ERR_UNSUPPORTED;
+}
+
+template <typename T, int D, int NR, int CPT, bool ROWS_SMEM>
+static pict_status_t launch_bicgstab_resident_as(KArgs<T>& a, bool trans, cudaStream_t st) {
+    return launch_resident<T>(k_bicgstab_resident<T, D, NR, CPT, ROWS_SMEM>, resident_smem<T, D, CPT, ROWS_SMEM>(2 * NR), a,
+                              trans, st);
+}
+
+template <typename T, int D, int NR>
+static pict_status_t launch_bicgstab_resident(KArgs<T>& a, bool trans, cudaStream_t st) {
+    const int cpt = resident_cpt(&a.dom);
+    if (cpt <= 1) return launch_bicgstab_resident_as<T, D, NR, 1, false>(a, trans, st);
+    if (cpt <= 2) return launch_bicgstab_resident_as<T, D, NR, 2, sizeof(T) == 8 || NR == 3>(a, trans, st);
+    if constexpr (sizeof(T) == 4 && NR <= 2)
+        if (cpt <= 4) return launch_bicgstab_resident_as<T, D, NR, 4, true>(a, trans, st);
+    return PICT_ERR_UNSUPPORTED;
+}
+
 template <typename KernelT>
 static int max_coresident(KernelT kernel) {
     int per_sm = 0;
@@ -2010,6 +2097,20 @@ static pict_status_t run_solve(const pict_domain_t* dom, const void* coef, const
         if (prm->use_bicg) {
             a.r = vec[0]; a.rw = vec[1]; a.p0 = vec[2]; a.p1 = vec[3]; a.v0 = vec[4]; a.v1 = vec[5]; a.t = vec[6];
             a.r1 = vec[7];  // null with the four-barrier kernel (7 vectors)
+            const bool few_small = dom->num_sims <= 8;
+            if (a.abs_crit == 0 && g_bicgstab_variant == 0 && (g_cluster_mode == 2 || (g_cluster_mode == 1 && few_small))) {
+                s = PICT_ERR_UNSUPPORTED;
+                if (nr == 1) s = launch_bicgstab_resident<T, D, 1>(a, TRANS, st);
+                else if (nr == 2) s = launch_bicgstab_resident<T, D, 2>(a, TRANS, st);
+                else if constexpr (D == 3) s = launch_bicgstab_resident<T, D, 3>(a, TRANS, st);
+                if (s == PICT_OK) {
+                    k_finish_info<<<1, 128, 0, st>>>(info, ninfo, ctrl);
+                    s = check_launch("finish_info");
+                    if (s) return s;
+                    continue;
+                }
+                if (s != PICT_ERR_UNSUPPORTED) return s;
+            }
             if (g_bicgstab_variant == 1 && a.abs_crit == 0 && nr <= 2)
                 kern = nr == 1 ? k_bicgstab2<T, D, 1, TRANS, 1> : k_bicgstab2<T, D, 2, TRANS, 1>;
             else if (g_bicgstab_variant == 2 && a.abs_crit == 0 && nr <= 2)
@@ -2025,7 +2126,8 @@ static pict_status_t run_solve(const pict_domain_t* dom, const void* coef, const
             // them while each cluster would pay its own per system
             const bool few_small = dom->num_sims <= 8 && dom->max_sim_cells <= 262144;
             if (g_cluster_mode == 2 || (g_cluster_mode == 1 && few_small)) {
-                s = launch_cg1_cluster<T, D, TRANS>(a, 16, st);
+                s = launch_cg1_resident<T, D>(a, TRANS, st);
+                if (s == PICT_ERR_UNSUPPORTED) s = launch_cg1_cluster<T, D, TRANS>(a, 16, st);
                 if (s == PICT_ERR_UNSUPPORTED) s = launch_cg1_cluster<T, D, TRANS>(a, 8, st);
                 if (s == PICT_OK) {
                     k_finish_info<<<1, 128, 0, st>>>(info, ninfo, ctrl);
