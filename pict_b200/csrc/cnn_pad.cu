@@ -23,39 +23,83 @@ struct MbTable {
     int64_t n[MB_MAX];  // cells per block (unpadded for the sources, padded for the outputs)
 };
 
+// Both kernels: a thread takes one cell of the map and walks its channels (stride gridDim.y), PAD_U at a time with
+// the loads ahead of the stores, so that a warp keeps PAD_U lines in flight; a pass is bound by HBM once enough bytes
+// are underway.  2x2 blocks of about 512^2 cells, 64 channels, FP32 (537 MB a pass): gather 161 -> 111 us (4.8 TB/s),
+// gather-sum 285 -> 111 us, whose reader list was walked anew for every channel.
+constexpr int PAD_U = 8;
+
 // out[ob][bc][pos] = src[sb][bc][loc] (0 where sb < 0) for padded cell j = (ob, pos) <- (sb, loc)
 template <typename T>
-__global__ void k_mb_pad_gather(int n, int bc, const int32_t* __restrict__ ob, const int32_t* __restrict__ pos,
-                                const int32_t* __restrict__ sb, const int32_t* __restrict__ loc, const MbTable<T> src,
-                                const MbTable<T> out) {
+__global__ void __launch_bounds__(PAD_THREADS) k_mb_pad_gather(int n, int bc, const int32_t* __restrict__ ob,
+                                                               const int32_t* __restrict__ pos,
+                                                               const int32_t* __restrict__ sb,
+                                                               const int32_t* __restrict__ loc, const MbTable<T> src,
+                                                               const MbTable<T> out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int o = ob[j], p = pos[j], s = sb[j], l = loc[j];
-    T* dst = out.p[o] + p;
+    T* __restrict__ dst = out.p[o] + p;
     const int64_t os = out.n[o];
+    const int step = gridDim.y;
     if (s < 0) {
-        for (int c = blockIdx.y; c < bc; c += gridDim.y) dst[(size_t)c * os] = T(0);
+        for (int c = blockIdx.y; c < bc; c += step) dst[(size_t)c * os] = T(0);
         return;
     }
-    const T* from = src.p[s] + l;
+    const T* __restrict__ from = src.p[s] + l;
     const int64_t ss = src.n[s];
-    for (int c = blockIdx.y; c < bc; c += gridDim.y) dst[(size_t)c * os] = from[(size_t)c * ss];
+    int c = blockIdx.y;
+    for (; c + (PAD_U - 1) * step < bc; c += PAD_U * step) {
+        T v[PAD_U];
+#pragma unroll
+        for (int u = 0; u < PAD_U; ++u) v[u] = from[(size_t)(c + u * step) * ss];
+#pragma unroll
+        for (int u = 0; u < PAD_U; ++u) dst[(size_t)(c + u * step) * os] = v[u];
+    }
+    for (; c < bc; c += step) dst[(size_t)c * os] = from[(size_t)c * ss];
 }
 
-// gsrc[sb][bc][loc] = sum over the readers k of source cell g = (sb, loc) of gout[ob_k][bc][pos_k]
+// gsrc[sb][bc][loc] = sum over the readers k of source cell g = (sb, loc) of gout[ob_k][bc][pos_k].  Away from the
+// connections a cell has one reader, the padded cell over itself, whose place is kept in registers; the others
+// follow in the list's order.
 template <typename T>
-__global__ void k_mb_pad_scatter_sum(int n, int bc, const int32_t* __restrict__ sb, const int32_t* __restrict__ loc,
-                                     const int32_t* __restrict__ ptr, const int32_t* __restrict__ rob,
-                                     const int32_t* __restrict__ rpos, const MbTable<T> gout, const MbTable<T> gsrc) {
+__global__ void __launch_bounds__(PAD_THREADS) k_mb_pad_scatter_sum(int n, int bc, const int32_t* __restrict__ sb,
+                                                                    const int32_t* __restrict__ loc,
+                                                                    const int32_t* __restrict__ ptr,
+                                                                    const int32_t* __restrict__ rob,
+                                                                    const int32_t* __restrict__ rpos,
+                                                                    const MbTable<T> gout, const MbTable<T> gsrc) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const int s = sb[g], l = loc[g], k0 = ptr[g], k1 = ptr[g + 1];
-    T* dst = gsrc.p[s] + l;
+    T* __restrict__ dst = gsrc.p[s] + l;
     const int64_t ss = gsrc.n[s];
-    for (int c = blockIdx.y; c < bc; c += gridDim.y) {
-        T acc = T(0);
-        for (int k = k0; k < k1; ++k) acc += gout.p[rob[k]][(size_t)c * gout.n[rob[k]] + rpos[k]];
-        dst[(size_t)c * ss] = acc;
+    const int step = gridDim.y;
+    if (k0 == k1) {
+        for (int c = blockIdx.y; c < bc; c += step) dst[(size_t)c * ss] = T(0);
+        return;
+    }
+    const int o = rob[k0];
+    const T* __restrict__ from = gout.p[o] + rpos[k0];
+    const int64_t os = gout.n[o];
+    int c = blockIdx.y;
+    for (; c + (PAD_U - 1) * step < bc; c += PAD_U * step) {
+        T v[PAD_U];
+#pragma unroll
+        for (int u = 0; u < PAD_U; ++u) v[u] = from[(size_t)(c + u * step) * os];
+        for (int k = k0 + 1; k < k1; ++k) {
+            const T* __restrict__ more = gout.p[rob[k]] + rpos[k];
+            const int64_t ms = gout.n[rob[k]];
+#pragma unroll
+            for (int u = 0; u < PAD_U; ++u) v[u] += more[(size_t)(c + u * step) * ms];
+        }
+#pragma unroll
+        for (int u = 0; u < PAD_U; ++u) dst[(size_t)(c + u * step) * ss] = v[u];
+    }
+    for (; c < bc; c += step) {
+        T v = from[(size_t)c * os];
+        for (int k = k0 + 1; k < k1; ++k) v += gout.p[rob[k]][(size_t)c * gout.n[rob[k]] + rpos[k]];
+        dst[(size_t)c * ss] = v;
     }
 }
 
