@@ -857,7 +857,8 @@ class Simulation:
                               total_time=self.total_time)
             domain.UpdateDomainData()
             B.CopyVelocityResultFromBlocks(domain)
-            domain.setPressureRHS(domain.velocityResult)
+            # a copy: the step's H/A assembly writes pressureRHS while other cells still read velocityResult
+            domain.setPressureRHS(domain.velocityResult.clone())
             domain.UpdateDomainData()
             B.SetupPressureMatrix(domain, time_step, flags, False)
             for pstep in range(self.pressure_non_ortho_steps if flags else 1):
