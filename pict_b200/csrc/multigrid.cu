@@ -89,6 +89,12 @@ __device__ __forceinline__ void mg_pdl_entry() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The parts of it, for kernels that first read what no kernel of the loop writes (tile and block tables, stencils:
+// complete before the loop's first kernel started, and a kernel's predecessor has waited for its own before this one
+// is launched), so that those reads overlap the predecessor.
+__device__ __forceinline__ void mg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void mg_pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ MgBlock mg_block(const pict_mg_level_t& L, int b) {
     const int* t = L.blocks + MG_BT * b;
     return MgBlock{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10]};
@@ -255,21 +261,20 @@ __device__ __forceinline__ double* mg_warp_part(double* part, int stride) {
     return part + ((size_t)blockIdx.x * MG_NW + (threadIdx.x >> 5)) * stride;
 }
 
-// b_c = R (b - A x_s) over the children of each coarse cell, x_s the pre-smoothed iterate: x0 (nu = 1) or
-// x1 = x0 + w (b - A x0) / diag (nu = 2), both from zero.  UPD (finest level): b = r - alpha q is formed on
-// the fly and stored to rn, and x += alpha p (x = alpha p when first) for the children.
+// b_c = R (b - A x0) over the children of each coarse cell, x0 the pre-smoothed iterate from zero (levels with one
+// smoothing sweep).  UPD (finest level): b = r - alpha q is formed on the fly and stored to rn, and x += alpha p
+// (x = alpha p when first) for the children.
 //
-// 2D tiles whose fine rows (children rows plus nu halo rows on each side) fit the stage (cap cells) take
-// the staged path: b and diag of those rows go to shared memory once, x_s is formed there, then each coarse
-// cell sums its children's residuals from there (a y-periodic wrap, nu = 1 only, forms x0 of that
-// neighbour from global).  nu = 2 is taken only where every tile of the level fits the stage.
+// 2D tiles whose fine rows (children rows plus one halo row on each side) fit the stage (cap cells) take
+// the staged path: b and diag of those rows go to shared memory once, x0 is formed there, then each coarse
+// cell sums its children's residuals from there (a y-periodic wrap forms x0 of that neighbour from global).
 template <typename T, int D, bool UPD>
 __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pict_mg_level_t C,
                                                            const T* __restrict__ r, const T* __restrict__ q,
                                                            T* __restrict__ rn, T* __restrict__ x,
                                                            const T* __restrict__ p, const double* __restrict__ sc,
                                                            int first, T* __restrict__ bc, T w, int cap,
-                                                           const double* __restrict__ dn, int nu) {
+                                                           const double* __restrict__ dn) {
     mg_pdl_entry();
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(C.tiles, blockIdx.x);
@@ -301,11 +306,11 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
     int ylo = 0, yhi = -1;
     if (D == 2) {
         const int lc0 = tl.s0 - Bc.off, lc1 = lc0 + tl.cnt - 1;
-        ylo = max(0, ((lc0 / Bc.sx) << Bc.shy) - nu);
-        yhi = min(Bf.sy - 1, ((lc1 / Bc.sx + 1) << Bc.shy) - 1 + nu);
+        ylo = max(0, ((lc0 / Bc.sx) << Bc.shy) - 1);
+        yhi = min(Bf.sy - 1, ((lc1 / Bc.sx + 1) << Bc.shy));
     }
     if (D == 2 && (yhi - ylo + 1) * sx <= cap) {
-        T* s_x0 = reinterpret_cast<T*>(mg_stage_raw);  // x_s: x0 (nu = 1) or x1 (nu = 2)
+        T* s_x0 = reinterpret_cast<T*>(mg_stage_raw);
         T* s_b = s_x0 + cap;
         T* s_d = s_b + cap;
         const int lo = Bf.off + ylo * sx, nh = (yhi - ylo + 1) * sx;
@@ -316,12 +321,8 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
         for (int e = threadIdx.x; e < nh; e += MG_TPB) {
             const int i = lo + e;
             const T bi = rhs(i), di = cf[i];
-            if (nu == 1) {
-                s_x0[e] = mg_x0(di, bi, w);
-                s_d[e] = di;
-            } else {
-                s_d[e] = (di != T(0)) ? mg_div(w, di) : T(0);  // w / diag
-            }
+            s_x0[e] = mg_x0(di, bi, w);
+            s_d[e] = di;
             s_b[e] = bi;
             if (UPD) {
                 const int par = (xx >> Bc.shx) + Bc.sx * (yy >> Bc.shy);
@@ -338,34 +339,6 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
             }
         }
         __syncthreads();
-        if (nu == 2) {
-            // x1 = x0 + w (b - A x0) / diag on the stage, x0 = (w / diag) b formed from the staged b and w / diag.
-            // Rows of the stage's edge whose outer neighbour row lies outside the stage get a value that no
-            // child reads (children rows are at least one row inside); the block's own edges are fixed faces.
-            auto x0s = [&](int c) { return s_d[c] * s_b[c]; };
-            int ey = (int)threadIdx.x / sx, ex = (int)threadIdx.x - ey * sx;
-            for (int e = threadIdx.x; e < nh; e += MG_TPB) {
-                const int i = lo + e, yg = ylo + ey;
-                const T di = cf[i], xi = x0s(e);
-                const T xm = ex > 0 ? x0s(e - 1) : x0s(e + sx - 1);
-                const T xp = ex + 1 < sx ? x0s(e + 1) : x0s(e - sx + 1);
-                const bool hm = ey > 0, hp = ey + 1 < nh / sx;
-                const T ym = hm ? x0s(e - sx) : T(0), yp = hp ? x0s(e + sx) : T(0);
-                T ax = di * xi;
-                ax += (ex > 0 || Bf.px) ? cf[(size_t)Nf + i] * xm : T(0);
-                ax += (ex + 1 < sx || Bf.px) ? cf[(size_t)2 * Nf + i] * xp : T(0);
-                ax += (yg > 0 && hm) ? cf[(size_t)3 * Nf + i] * ym : T(0);
-                ax += (yg + 1 < Bf.sy && hp) ? cf[(size_t)4 * Nf + i] * yp : T(0);
-                s_x0[e] = xi + s_d[e] * (s_b[e] - ax);
-                ex += dr;
-                ey += dq;
-                if (ex >= sx) {
-                    ex -= sx;
-                    ++ey;
-                }
-            }
-            __syncthreads();
-        }
         auto far = [&](int xq, int yq) -> T {
             const int j = Bf.off + xq + sx * yq;
             return mg_x0(cf[j], rhs(j), w);
@@ -387,7 +360,7 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
                 const T xp = xs + 1 < sx ? s_x0[c + 1] : s_x0[c - sx + 1];
                 const T ym = ys > 0 ? s_x0[c - sx] : (Bf.py ? far(xs, Bf.sy - 1) : T(0));
                 const T yp = ys + 1 < Bf.sy ? s_x0[c + sx] : (Bf.py ? far(xs, 0) : T(0));
-                T ax = (nu == 2 ? cf[i] : s_d[c]) * xi;
+                T ax = s_d[c] * xi;
                 ax += (xs > 0 || Bf.px) ? cf[(size_t)Nf + i] * xm : T(0);
                 ax += (xs + 1 < sx || Bf.px) ? cf[(size_t)2 * Nf + i] * xp : T(0);
                 ax += (ys > 0 || Bf.py) ? cf[(size_t)3 * Nf + i] * ym : T(0);
@@ -452,24 +425,18 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
     }
 }
 
-// post-smoothing with the coarse correction: x' = x_s + s P e_c (formed on the fly, also for the
-// neighbours), then nu damped-Jacobi sweeps x <- x + w (b - A x) / diag.  x_s is the pre-smoothed iterate
-// of the restriction, recomputed here: x0 = w b / diag (nu = 1) or x1 = x0 + w (b - A x0) / diag (nu = 2).
-// DOT (finest level): per-warp partials of b.out, b.b, sum(out), sum(b).
+// post-smoothing with the coarse correction (levels with one smoothing sweep): x' = x0 + s P e_c (formed on the fly,
+// also for the neighbours; x0 = w b / diag, the pre-smoothed iterate, recomputed here), then one damped-Jacobi sweep
+// x' + w (b - A x') / diag.  DOT (finest level): per-warp partials of b.out, b.b, sum(out), sum(b).
 //
-// 2D tiles take a staged path where their rows plus the halo rows fit the stage.
-// nu = 1 (cap cells per array): x' of every cell of [first - sx, last + sx] is formed once into shared memory (with b and diag),
-// then the stencil reads its neighbours there; a y-periodic wrap reaches outside the stage and forms x'
-// of that neighbour from global memory.  nu = 2: b and diag of [first - 3 sx, last + 3 sx] are staged,
-// x1 (the pre-smoothed iterate) of [first - 2 sx, last + 2 sx], then the first post sweep of
-// [first - sx, last + sx] (x' formed from x1 and e_c on the fly), then the second sweep of the tile's
-// cells, in four arrays of 3 cap / 4 cells; taken only where every tile of the level fits (no y-periodic
-// wrap).
+// 2D tiles whose rows plus one halo row on each side fit the stage (cap cells per array) form x' of every cell of
+// [first - sx, last + sx] once into shared memory (with b and diag), then the stencil reads its neighbours there; a
+// y-periodic wrap reaches outside the stage and forms x' of that neighbour from global memory.
 template <typename T, int D, bool DOT>
 __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pict_mg_level_t C, const int32_t* tiles,
                                                           const T* __restrict__ bv, const T* __restrict__ ec,
                                                           T* __restrict__ out, T s, T w, double* __restrict__ part,
-                                                          int cap, const double* __restrict__ dn, int nu) {
+                                                          int cap, const double* __restrict__ dn) {
     mg_pdl_entry();
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(tiles, blockIdx.x);
@@ -479,102 +446,7 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
     const int N = F.num_cells;
     double a = 0.0, c2 = 0.0, sz = 0.0, sr = 0.0;
     const int sx = Bf.sx;
-    const int cap4 = (3 * cap) / 4;  // four arrays in the shared memory of three of `cap` cells
-    if (D == 2 && nu == 2 && tl.cnt + 6 * sx <= cap4) {
-        T* s_x = reinterpret_cast<T*>(mg_stage_raw);  // x0, then the first post sweep
-        T* s_b = s_x + cap4;
-        T* s_r = s_b + cap4;                           // w / diag
-        T* s_y = s_r + cap4;                           // x1, then x' = x1 + s P e_c
-        const int nf = sx * Bf.sy;
-        const int lo = max(Bf.off, tl.s0 - 3 * sx), hi = min(Bf.off + nf, tl.s0 + tl.cnt + 3 * sx);
-        for (int e = threadIdx.x; e < hi - lo; e += MG_TPB) {
-            const T d = cf[lo + e], bb = bv[lo + e];
-            const T r = (d != T(0)) ? mg_div(w, d) : T(0);
-            s_b[e] = bb;
-            s_r[e] = r;
-            s_x[e] = r * bb;
-        }
-        __syncthreads();
-        // one damped-Jacobi sweep over the global cells [g0, g1): dst = src + (w / diag) (b - A src), src and dst
-        // on the stage; neighbours outside the block are fixed faces (no y-periodic wrap on this path)
-        auto sweep = [&](int g0, int g1, const T* src, T* dst) {
-            const int dq = MG_TPB / sx, dr = MG_TPB - dq * sx;
-            int l = g0 - Bf.off + (int)threadIdx.x;
-            int y = l / sx, x = l - y * sx;
-            for (int i = g0 + (int)threadIdx.x; i < g1; i += MG_TPB) {
-                const int c = i - lo;
-                const T xi = src[c];
-                const T xm = x > 0 ? src[c - 1] : src[c + sx - 1];
-                const T xp = x + 1 < sx ? src[c + 1] : src[c - sx + 1];
-                const T ym = y > 0 ? src[c - sx] : T(0);
-                const T yp = y + 1 < Bf.sy ? src[c + sx] : T(0);
-                T acc = cf[i] * xi;
-                acc += (x > 0 || Bf.px) ? cf[(size_t)N + i] * xm : T(0);
-                acc += (x + 1 < sx || Bf.px) ? cf[(size_t)2 * N + i] * xp : T(0);
-                acc += y > 0 ? cf[(size_t)3 * N + i] * ym : T(0);
-                acc += y + 1 < Bf.sy ? cf[(size_t)4 * N + i] * yp : T(0);
-                dst[c] = xi + s_r[c] * (s_b[c] - acc);
-                x += dr;
-                y += dq;
-                if (x >= sx) {
-                    x -= sx;
-                    ++y;
-                }
-            }
-        };
-        const int a1 = max(Bf.off, tl.s0 - 2 * sx), b1 = min(Bf.off + nf, tl.s0 + tl.cnt + 2 * sx);
-        const int a2 = max(Bf.off, tl.s0 - sx), b2 = min(Bf.off + nf, tl.s0 + tl.cnt + sx);
-        sweep(a1, b1, s_x, s_y);  // x1: the pre-smoothed iterate of the restriction
-        __syncthreads();
-        {  // x' = x1 + s P e_c
-            const int dq = MG_TPB / sx, dr = MG_TPB - dq * sx;
-            int l = a1 - Bf.off + (int)threadIdx.x;
-            int y = l / sx, x = l - y * sx;
-            for (int i = a1 + (int)threadIdx.x; i < b1; i += MG_TPB) {
-                s_y[i - lo] += s * ec[Bc.off + (x >> Bc.shx) + Bc.sx * (y >> Bc.shy)];
-                x += dr;
-                y += dq;
-                if (x >= sx) {
-                    x -= sx;
-                    ++y;
-                }
-            }
-        }
-        __syncthreads();
-        sweep(a2, b2, s_y, s_x);  // first post sweep
-        __syncthreads();
-        // second post sweep of the tile's cells
-        const int dq = MG_TPB / sx, dr = MG_TPB - dq * sx;
-        int l = tl.s0 - Bf.off + (int)threadIdx.x;
-        int y = l / sx, x = l - y * sx;
-        for (int k = threadIdx.x; k < tl.cnt; k += MG_TPB) {
-            const int i = tl.s0 + k, c = i - lo;
-            const T xi = s_x[c], bi = s_b[c];
-            const T xm = x > 0 ? s_x[c - 1] : s_x[c + sx - 1];
-            const T xp = x + 1 < sx ? s_x[c + 1] : s_x[c - sx + 1];
-            const T ym = y > 0 ? s_x[c - sx] : T(0);
-            const T yp = y + 1 < Bf.sy ? s_x[c + sx] : T(0);
-            T acc = cf[i] * xi;
-            acc += (x > 0 || Bf.px) ? cf[(size_t)N + i] * xm : T(0);
-            acc += (x + 1 < sx || Bf.px) ? cf[(size_t)2 * N + i] * xp : T(0);
-            acc += y > 0 ? cf[(size_t)3 * N + i] * ym : T(0);
-            acc += y + 1 < Bf.sy ? cf[(size_t)4 * N + i] * yp : T(0);
-            const T zi = xi + s_r[c] * (bi - acc);
-            out[i] = zi;
-            if (DOT) {
-                a += (double)bi * (double)zi;
-                c2 += (double)bi * (double)bi;
-                sz += (double)zi;
-                sr += (double)bi;
-            }
-            x += dr;
-            y += dq;
-            if (x >= sx) {
-                x -= sx;
-                ++y;
-            }
-        }
-    } else if (D == 2 && tl.cnt + 2 * sx <= cap) {
+    if (D == 2 && tl.cnt + 2 * sx <= cap) {
         T* s_x = reinterpret_cast<T*>(mg_stage_raw);
         T* s_b = s_x + cap;
         T* s_d = s_b + cap;
@@ -690,6 +562,251 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
 }
 
 // ---------------------------------------------------------------------------------------------
+// The two-sweep tile kernels (2D, no y-periodic block).  A CTA of MG2_TPB threads holds the rows of its tile and the
+// halo rows of the sweeps in shared memory: w / diag and the +x and +y couplings (the operator is symmetric, so a
+// cell's -x and -y couplings are its neighbours' and five coefficients become three), the right-hand side and two
+// iterates.  The stencil is staged before the wait on the predecessor (mg_pdl_wait), so what is left of a kernel's own
+// chain is one read of the right-hand side and the sweeps in shared memory.  A coupling across a fixed face is 0, which
+// masks its term: -x of the first cell of a row reads the +x coupling of the row's last cell, the periodic one or 0.
+//
+// What bounds them: on few systems the latency of this chain (a level is a few CTAs), on many the shared-memory
+// reads of the sweeps over tile and halo.  Per launch of the finest level, before (256 threads, everything but b and the
+// iterates read through L1 after the wait) -> now: 16 cavities (272k cells) prolongation 10.9 -> 8.3 us, restriction
+// 16.3 -> 7.8; 256 cavities (4.34 M) prolongation 57 -> 48..55, restriction 60 -> 44..51 (69 and 57 when staged).
+// ---------------------------------------------------------------------------------------------
+// STAGED keeps the couplings in shared memory too (512 threads, two CTAs on an SM); otherwise they are read through L1
+// where they are used (256 threads, more CTAs on an SM).
+constexpr int MG_TILE = 512;                  // cells of a coarse level's work tile (multigrid.py TILE_CELLS)
+constexpr int MG2_WAVES = 4;                  // CTAs per SM up to which a launch counts as one wave
+constexpr size_t MG2_MAX_SMEM = 192 * 1024;  // of one two-sweep CTA (FP64 stages of the widest blocks)
+
+// (A v) at stage cell c (column x of rows of sx, stage of nst cells).  The diagonal term is kept beside the others and
+// not folded into a (1 - w) v, so that what is left of a constant v cancels here and is not carried through the sweeps.
+template <typename T>
+__device__ __forceinline__ T mg2_apply(const T* v, const T* d, const T* cx, const T* cy, int c, int x, int sx, int nst) {
+    const int m = x > 0 ? c - 1 : c + sx - 1, p = x + 1 < sx ? c + 1 : c - sx + 1;
+    T acc = d[c] * v[c];
+    acc += cx[m] * v[m];
+    acc += cx[c] * v[p];
+    if (c >= sx) acc += cy[c - sx] * v[c - sx];
+    if (c + sx < nst) acc += cy[c] * v[c + sx];
+    return acc;
+}
+
+// one damped-Jacobi sweep there: v + r (b - A v) with r = w / diag
+template <typename T>
+__device__ __forceinline__ T mg2_sweep(const T* v, const T* b, const T* r, const T* d, const T* cx, const T* cy, int c, int x,
+                                       int sx, int nst) {
+    return v[c] + r[c] * (b[c] - mg2_apply(v, d, cx, cy, c, x, sx, nst));
+}
+
+template <bool STAGED>
+struct Mg2 {
+    static constexpr int threads = STAGED ? 512 : 256;
+};
+
+// stages w / diag and (STAGED) the diagonal and the couplings of the cells [lo, lo + nst)
+template <typename T, bool STAGED>
+__device__ __forceinline__ void mg2_stage_stencil(const T* __restrict__ cf, int N, int lo, int nst, T w, T* r, T* dd, T* cx,
+                                                  T* cy) {
+    for (int e = threadIdx.x; e < nst; e += Mg2<STAGED>::threads) {
+        const T d = cf[lo + e];
+        if (STAGED) {
+            dd[e] = d;
+            cx[e] = cf[(size_t)2 * N + lo + e];
+            cy[e] = cf[(size_t)4 * N + lo + e];
+        }
+        r[e] = (d != T(0)) ? mg_div(w, d) : T(0);
+    }
+}
+
+// b_c = R (b - A x1) over the children of each coarse cell, x1 the pre-smoothed iterate after two sweeps from zero.
+// UPD as k_mg_restrict.  Stage: the children's rows and two halo rows on each side (three arrays of `cap` cells, three more
+// when STAGED).
+template <typename T, bool UPD, bool STAGED>
+__global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_restrict2(pict_mg_level_t F, pict_mg_level_t C, const T* __restrict__ r,
+                                                             const T* __restrict__ q, T* __restrict__ rn, T* __restrict__ x,
+                                                             const T* __restrict__ p, const double* __restrict__ sc, int first,
+                                                             T* __restrict__ bc, T w, int cap) {
+    constexpr int MG2_TPB = Mg2<STAGED>::threads;
+    extern __shared__ __align__(16) unsigned char mg_stage_raw[];
+    const MgTile tl = mg_tile(C.tiles, blockIdx.x);
+    const MgBlock Bc = mg_block(C, tl.blk), Bf = mg_block(F, tl.blk);
+    const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
+    const int Nf = F.num_cells, sx = Bf.sx;
+    const int lc0 = tl.s0 - Bc.off, lc1 = lc0 + tl.cnt - 1;
+    const int ylo = max(0, ((lc0 / Bc.sx) << Bc.shy) - 2);
+    const int yhi = min(Bf.sy - 1, ((lc1 / Bc.sx + 1) << Bc.shy) + 1);
+    const int lo = Bf.off + ylo * sx, nst = (yhi - ylo + 1) * sx;
+    if (nst > cap) return;  // a tile table that does not keep the level's promise (sweeps = 2) stays in bounds
+    T* s_x = reinterpret_cast<T*>(mg_stage_raw);  // x1
+    T* s_b = s_x + cap;
+    T* s_r = s_b + cap;
+    mg2_stage_stencil<T, STAGED>(cf, Nf, lo, nst, w, s_r, s_r + cap, s_r + 2 * cap, s_r + 3 * cap);
+    const T* s_d = STAGED ? s_r + cap : cf + lo;
+    const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * Nf + lo;
+    const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * Nf + lo;
+    const int dq = MG2_TPB / sx, dr = MG2_TPB - dq * sx;
+    const int y0 = (int)threadIdx.x / sx, x0 = (int)threadIdx.x - y0 * sx;
+    mg_pdl_wait();
+    mg_pdl_next();
+    const bool pend = UPD && mg_pending(sc, tl.sys);
+    if (mg_done(sc, tl.sys) && !pend) return;
+    const T al = UPD ? (T)sc[MG_SC * tl.sys + 1] : T(0);
+    {
+        int xx = x0, yy = y0 + ylo;
+        for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
+            const int i = lo + e;
+            const T bi = UPD ? r[i] - al * q[i] : r[i];
+            if (UPD) {
+                const int par = (xx >> Bc.shx) + Bc.sx * (yy >> Bc.shy);
+                if (par >= lc0 && par <= lc1) {
+                    rn[i] = bi;
+                    x[i] = first ? al * p[i] : x[i] + al * p[i];
+                }
+                xx += dr;
+                yy += dq;
+                if (xx >= sx) {
+                    xx -= sx;
+                    ++yy;
+                }
+            }
+            s_b[e] = bi;
+        }
+    }
+    if (pend) return;  // converged at this iteration: only the update of its cells
+    __syncthreads();
+    {   // x1 = x0 + w (b - A x0) / diag with x0 = (w / diag) b formed from the stage.  Cells of the outermost rows whose
+        // outer neighbour row is outside the stage get a value that no child reads.
+        int xx = x0;
+        for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
+            const int m = xx > 0 ? e - 1 : e + sx - 1, pp = xx + 1 < sx ? e + 1 : e - sx + 1;
+            const T rc = s_r[e], xi = rc * s_b[e];
+            T acc = s_d[e] * xi;
+            acc += s_cx[m] * (s_r[m] * s_b[m]);
+            acc += s_cx[e] * (s_r[pp] * s_b[pp]);
+            if (e >= sx) acc += s_cy[e - sx] * (s_r[e - sx] * s_b[e - sx]);
+            if (e + sx < nst) acc += s_cy[e] * (s_r[e + sx] * s_b[e + sx]);
+            s_x[e] = xi + rc * (s_b[e] - acc);
+            xx += dr;
+            if (xx >= sx) xx -= sx;
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < tl.cnt; k += MG2_TPB) {
+        const int l = lc0 + k, Y = l / Bc.sx, X = l - Y * Bc.sx;
+        T acc = T(0);
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+            const int dx = ch & 1, dy = ch >> 1;
+            const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy;
+            if ((dx && !Bc.shx) || (dy && !Bc.shy) || xs >= sx || ys >= Bf.sy) continue;
+            const int c = (ys - ylo) * sx + xs;
+            acc += s_b[c] - mg2_apply(s_x, s_d, s_cx, s_cy, c, xs, sx, nst);
+        }
+        bc[tl.s0 + k] = acc;
+    }
+}
+
+// post-smoothing with the coarse correction, two sweeps: x1 (the pre-smoothed iterate of the restriction, recomputed)
+// on the tile and two halo rows, x' = x1 + s P e_c, the first sweep on the tile and one halo row, the second on the
+// tile.  DOT (finest level): partials of out.b, b.b, sum(out), sum(b) in the tile's MG_NW slots.  Stage: the tile and
+// three halo rows on each side (four arrays of
+// `cap` cells, three more when STAGED).
+template <typename T, bool DOT, bool STAGED>
+__global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_prolong2(pict_mg_level_t F, pict_mg_level_t C, const int32_t* tiles,
+                                                            const T* __restrict__ bv, const T* __restrict__ ec,
+                                                            T* __restrict__ out, T s, T w, double* __restrict__ part, int cap,
+                                                            const double* __restrict__ sc) {
+    constexpr int MG2_TPB = Mg2<STAGED>::threads;
+    extern __shared__ __align__(16) unsigned char mg_stage_raw[];
+    __shared__ double s_red[MG2_TPB / 32][4];
+    const MgTile tl = mg_tile(tiles, blockIdx.x);
+    const MgBlock Bf = mg_block(F, tl.blk), Bc = mg_block(C, tl.blk);
+    const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
+    const int N = F.num_cells, sx = Bf.sx, nf = sx * Bf.sy;
+    const int lo = max(Bf.off, tl.s0 - 3 * sx), hi = min(Bf.off + nf, tl.s0 + tl.cnt + 3 * sx), nst = hi - lo;
+    if (nst > cap) return;  // as k_mg_restrict2
+    T* s_x = reinterpret_cast<T*>(mg_stage_raw);  // x0, then the first post sweep
+    T* s_y = s_x + cap;                           // s P e_c, then x'
+    T* s_b = s_y + cap;
+    T* s_r = s_b + cap;
+    mg2_stage_stencil<T, STAGED>(cf, N, lo, nst, w, s_r, s_r + cap, s_r + 2 * cap, s_r + 3 * cap);
+    const T* s_d = STAGED ? s_r + cap : cf + lo;
+    const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * N + lo;
+    const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * N + lo;
+    const int dq = MG2_TPB / sx, dr = MG2_TPB - dq * sx;
+    mg_pdl_wait();
+    mg_pdl_next();
+    if (mg_done(sc, tl.sys)) return;
+    {
+        const int l = lo - Bf.off + (int)threadIdx.x;
+        int y = l / sx, x = l - y * sx;
+        for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
+            const T b = bv[lo + e];
+            s_y[e] = s * ec[Bc.off + (x >> Bc.shx) + Bc.sx * (y >> Bc.shy)];
+            s_b[e] = b;
+            s_x[e] = s_r[e] * b;  // written by this thread
+            x += dr;
+            y += dq;
+            if (x >= sx) {
+                x -= sx;
+                ++y;
+            }
+        }
+    }
+    __syncthreads();
+    // stage cells [c0, c1): f(stage cell, its column)
+    auto cells = [&](int c0, int c1, auto&& f) {
+        int x = (lo - Bf.off + c0 + (int)threadIdx.x) % sx;
+        for (int c = c0 + (int)threadIdx.x; c < c1; c += MG2_TPB) {
+            f(c, x);
+            x += dr;
+            if (x >= sx) x -= sx;
+        }
+    };
+    const int t0 = tl.s0 - lo, t1 = t0 + tl.cnt;
+    cells(max(0, t0 - 2 * sx), min(nst, t1 + 2 * sx),
+          [&](int c, int x) { s_y[c] += mg2_sweep(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+    __syncthreads();
+    cells(max(0, t0 - sx), min(nst, t1 + sx),
+          [&](int c, int x) { s_x[c] = mg2_sweep(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+    __syncthreads();
+    double a = 0.0, c2 = 0.0, sz = 0.0, sr = 0.0;
+    cells(t0, t1, [&](int c, int x) {
+        const T zi = mg2_sweep(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst);
+        out[lo + c] = zi;
+        if (DOT) {
+            const double bi = (double)s_b[c];
+            a += bi * (double)zi;
+            c2 += bi * bi;
+            sz += (double)zi;
+            sr += bi;
+        }
+    });
+    if (DOT) {
+        a = mg_warp_sum(a);
+        c2 = mg_warp_sum(c2);
+        sz = mg_warp_sum(sz);
+        sr = mg_warp_sum(sr);
+        const int wp = threadIdx.x >> 5;
+        if ((threadIdx.x & 31) == 0) {
+            s_red[wp][0] = a;
+            s_red[wp][1] = c2;
+            s_red[wp][2] = sz;
+            s_red[wp][3] = sr;
+        }
+        __syncthreads();
+        if (threadIdx.x < 4 * MG_NW) {  // the warps' sums in the tile's MG_NW slots
+            const int k = threadIdx.x & 3, j = threadIdx.x >> 2;
+            double v = 0.0;
+            for (int u = j; u < MG2_TPB / 32; u += MG_NW) v += s_red[u][k];
+            part[((size_t)blockIdx.x * MG_NW + j) * 4 + k] = v;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // The V-cycle below a size cutoff in one launch: one CTA per block runs the levels lv[0..n-1] of its
 // block (nu pre-smoothing sweeps from zero and restriction down to the coarsest, `sweeps` damped-Jacobi
 // sweeps from zero and mean removal on the coarsest, prolongation and nu post-smoothing sweeps up) with every level's right-hand side, iterate and
@@ -708,28 +825,50 @@ struct MgSub {
 };
 
 // shared memory of the sub-cycle: b, x and the 2D+1 stencil rows of every level (this block's cells)
-// and one scratch vector
+// and two scratch vectors
 static size_t mg_sub_smem(const pict_mg_level_t* lv, int n, size_t esz) {
     const size_t K = 2 * (size_t)lv[0].dims + 1;
-    size_t c = (size_t)lv[0].max_block_cells;
+    size_t c = 2 * (size_t)lv[0].max_block_cells;
     for (int k = 0; k < n; ++k) c += (2 + K) * (size_t)lv[k].max_block_cells;
     return c * esz;
+}
+
+// coordinates of a cell of a block of at most 2^20 cells without an integer division: (e + 1/2) / sx is at least
+// 1 / (2 sx) away from an integer, more than the rounding of the product while e < 2^21
+struct MgCell {
+    float rx, ry;
+    __device__ __forceinline__ explicit MgCell(const MgBlock& B) : rx(1.0f / (float)B.sx), ry(1.0f / (float)B.sy) {}
+    template <int D>
+    __device__ __forceinline__ void at(const MgBlock& B, int e, int& x, int& y, int& z) const {
+        const int t = (int)(((float)e + 0.5f) * rx);
+        x = e - t * B.sx;
+        z = D > 2 ? (int)(((float)t + 0.5f) * ry) : 0;
+        y = t - z * B.sy;
+    }
+};
+
+// off-diagonal part of A v at a cell of a sub-cycle level in shared memory (rows of n cells)
+template <typename T, int D>
+__device__ __forceinline__ T mg_sub_off(const MgBlock& B, int n, const T* sc, const T* v, int e, int x, int y, int z) {
+    T acc = T(0);
+#pragma unroll
+    for (int f = 0; f < 2 * D; ++f) {
+        const int j = mg_nbr(B, x, y, z, f);
+        if (j >= 0) acc += sc[(f + 1) * n + e] * v[j - B.off];
+    }
+    return acc;
 }
 
 // one damped-Jacobi sweep of a sub-cycle level in shared memory: xd = xs + w (b - A xs) / diag
 template <typename T, int D>
 __device__ __forceinline__ void mg_sub_sweep(const MgBlock& B, int n, const T* sc, const T* sb, const T* xs, T* xd,
                                              T w) {
+    const MgCell cell(B);
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         int x, y, z;
-        mg_unflatten(B, e, x, y, z);
-        T acc = sc[e] * xs[e];
-#pragma unroll
-        for (int f = 0; f < 2 * D; ++f) {
-            const int j = mg_nbr(B, x, y, z, f);
-            if (j >= 0) acc += sc[(f + 1) * n + e] * xs[j - B.off];
-        }
+        cell.at<D>(B, e, x, y, z);
         const T d = sc[e];
+        const T acc = d * xs[e] + mg_sub_off<T, D>(B, n, sc, xs, e, x, y, z);
         xd[e] = xs[e] + ((d != T(0)) ? mg_div(w * (sb[e] - acc), d) : T(0));
     }
 }
@@ -738,15 +877,11 @@ template <typename T, int D>
 __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T* __restrict__ bin,
                                                                 T* __restrict__ xout, T w, T sp, int sweeps,
                                                                 const double* __restrict__ dn, int nu) {
-    mg_pdl_entry();
     constexpr int K = 2 * D + 1;
     extern __shared__ __align__(16) unsigned char mg_sub_raw[];
     T* sm = reinterpret_cast<T*>(mg_sub_raw);
     __shared__ int s_off[MG_SUB_LEVELS + 1];
-    __shared__ double s_red[32];
-    __shared__ double s_mean;
     const int b = blockIdx.x;
-    if (mg_done(dn, mg_block(S.lv[0], b).sys)) return;
     if (threadIdx.x == 0) {
         int o = 0;
         for (int k = 0; k < S.n; ++k) {
@@ -757,21 +892,27 @@ __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T
         s_off[S.n] = o;
     }
     __syncthreads();
-    T* scr = sm + s_off[S.n];
-    // level k of this block: b at sm + s_off[k], x after it, then the stencil rows
+    // level k of this block: b at sm + s_off[k], x after it, then the stencil rows (staged before the wait)
     for (int k = 0; k < S.n; ++k) {
         const pict_mg_level_t& L = S.lv[k];
         const MgBlock B = mg_block(L, b);
         const int n = B.sx * B.sy * B.sz;
         const T* __restrict__ cf = reinterpret_cast<const T*>(L.coef);
         T* sc = sm + s_off[k] + 2 * n;
-        for (int f = 0; f < K; ++f)
-            for (int e = threadIdx.x; e < n; e += blockDim.x) sc[f * n + e] = cf[(size_t)f * L.num_cells + B.off + e];
-        if (k == 0)
-            for (int e = threadIdx.x; e < n; e += blockDim.x) sm[s_off[0] + e] = bin[B.off + e];
+        for (int e = threadIdx.x; e < n; e += blockDim.x)
+#pragma unroll
+            for (int f = 0; f < K; ++f) sc[f * n + e] = cf[(size_t)f * L.num_cells + B.off + e];
     }
+    const MgBlock B0 = mg_block(S.lv[0], b);
+    const int n0 = B0.sx * B0.sy * B0.sz;
+    T* const scr = sm + s_off[S.n];
+    T* const scr2 = scr + n0;
+    mg_pdl_wait();
+    mg_pdl_next();
+    if (mg_done(dn, B0.sys)) return;
+    for (int e = threadIdx.x; e < n0; e += blockDim.x) sm[s_off[0] + e] = bin[B0.off + e];
     __syncthreads();
-    // down: x0 = w b / diag (kept in the level's x), b_c = R (b - A x0)
+    // down: x0 = w b / diag, with nu = 2 a second sweep, kept in the level's x; b_c = R (b - A x)
     for (int k = 0; k + 1 < S.n; ++k) {
         const MgBlock Bf = mg_block(S.lv[k], b), Bc = mg_block(S.lv[k + 1], b);
         const int nf = Bf.sx * Bf.sy * Bf.sz, nc = Bc.sx * Bc.sy * Bc.sz;
@@ -779,82 +920,83 @@ __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T
         T* sx = sb + nf;
         const T* sc = sx + nf;
         T* sbc = sm + s_off[k + 1];
-        for (int e = threadIdx.x; e < nf; e += blockDim.x) sx[e] = mg_x0(sc[e], sb[e], w);
+        T* x0 = nu == 2 ? scr : sx;
+        for (int e = threadIdx.x; e < nf; e += blockDim.x) x0[e] = mg_x0(sc[e], sb[e], w);
         __syncthreads();
-        if (nu == 2) {  // second pre-smoothing sweep (through the scratch vector)
-            mg_sub_sweep<T, D>(Bf, nf, sc, sb, sx, scr, w);
-            __syncthreads();
-            for (int e = threadIdx.x; e < nf; e += blockDim.x) sx[e] = scr[e];
+        if (nu == 2) {
+            mg_sub_sweep<T, D>(Bf, nf, sc, sb, scr, sx, w);
             __syncthreads();
         }
+        const MgCell cell(Bc);
         for (int E = threadIdx.x; E < nc; E += blockDim.x) {
             int X, Y, Z;
-            mg_unflatten(Bc, E, X, Y, Z);
+            cell.at<D>(Bc, E, X, Y, Z);
             T acc = T(0);
+#pragma unroll
             for (int c = 0; c < (1 << D); ++c) {
                 const int dx = c & 1, dy = (c >> 1) & 1, dz = (c >> 2) & 1;
                 if ((dx && !Bc.shx) || (dy && !Bc.shy) || (dz && !Bc.shz)) continue;
                 const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy, zs = (Z << Bc.shz) + dz;
                 if (xs >= Bf.sx || ys >= Bf.sy || zs >= Bf.sz) continue;
                 const int il = xs + Bf.sx * (ys + Bf.sy * zs);
-                T ax = sc[il] * sx[il];
-#pragma unroll
-                for (int f = 0; f < 2 * D; ++f) {
-                    const int j = mg_nbr(Bf, xs, ys, zs, f);
-                    if (j >= 0) ax += sc[(f + 1) * nf + il] * sx[j - Bf.off];
-                }
-                acc += sb[il] - ax;
+                acc += sb[il] - (sc[il] * sx[il] + mg_sub_off<T, D>(Bf, nf, sc, sx, il, xs, ys, zs));
             }
             sbc[E] = acc;
         }
         __syncthreads();
     }
-    // coarsest: sweeps from zero (ping-pong between x and the scratch vector), then mean removal
+    // coarsest: sweeps from zero, then mean removal.  At most 32 cells are swept by one warp, which needs no block
+    // barrier between its sweeps; larger ones by the block (ping-pong between x and the scratch vector).
     {
         const MgBlock B = mg_block(S.lv[S.n - 1], b);
         const int n = B.sx * B.sy * B.sz;
         T* sb = sm + s_off[S.n - 1];
         T* const xa = sb + n;
         const T* sc = xa + n;
-        for (int e = threadIdx.x; e < n; e += blockDim.x) xa[e] = mg_x0(sc[e], sb[e], w);
-        __syncthreads();
-        int cur = 0;
-        for (int it = 1; it < sweeps; ++it) {
-            const T* xs = cur ? scr : xa;
-            T* xd = cur ? xa : scr;
-            for (int e = threadIdx.x; e < n; e += blockDim.x) {
-                int x, y, z;
-                mg_unflatten(B, e, x, y, z);
-                T acc = sc[e] * xs[e];
-#pragma unroll
-                for (int f = 0; f < 2 * D; ++f) {
-                    const int j = mg_nbr(B, x, y, z, f);
-                    if (j >= 0) acc += sc[(f + 1) * n + e] * xs[j - B.off];
+        if (n <= 32) {
+            if (threadIdx.x < 32) {
+                const int e = threadIdx.x;
+                const bool in = e < n;
+                int x = 0, y = 0, z = 0;
+                if (in) MgCell(B).at<D>(B, e, x, y, z);
+                const T d = in ? sc[e] : T(0), be = in ? sb[e] : T(0);
+                T v = mg_x0(d, be, w);
+                for (int it = 1; it < sweeps; ++it) {
+                    if (in) xa[e] = v;
+                    __syncwarp();
+                    const T off = in ? mg_sub_off<T, D>(B, n, sc, xa, e, x, y, z) : T(0);
+                    __syncwarp();
+                    v += (d != T(0)) ? mg_div(w * (be - (d * v + off)), d) : T(0);
                 }
-                const T d = sc[e];
-                xd[e] = xs[e] + ((d != T(0)) ? mg_div(w * (sb[e] - acc), d) : T(0));
+                const double m = mg_warp_sum(in ? (double)v : 0.0) / (double)n;
+                if (in) xa[e] = v - (T)m;
             }
+        } else {
+            __shared__ double s_red[MG_SUB_THREADS / 32];
+            for (int e = threadIdx.x; e < n; e += blockDim.x) xa[e] = mg_x0(sc[e], sb[e], w);
             __syncthreads();
-            cur ^= 1;
-        }
-        const T* xr = cur ? scr : xa;
-        double acc = 0.0;
-        for (int e = threadIdx.x; e < n; e += blockDim.x) acc += (double)xr[e];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
+            T* xs = xa;
+            T* xd = scr;
+            for (int it = 1; it < sweeps; ++it) {
+                mg_sub_sweep<T, D>(B, n, sc, sb, xs, xd, w);
+                __syncthreads();
+                T* t = xs;
+                xs = xd;
+                xd = t;
+            }
+            double acc = 0.0;
+            for (int e = threadIdx.x; e < n; e += blockDim.x) acc += (double)xs[e];
+            acc = mg_warp_sum(acc);
+            if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
+            __syncthreads();
             double v = 0.0;
-            for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) v += s_red[wv];
-            s_mean = v / (double)n;
+            for (int u = 0; u < MG_SUB_THREADS / 32; ++u) v += s_red[u];
+            const T m = (T)(v / (double)n);
+            for (int e = threadIdx.x; e < n; e += blockDim.x) xa[e] = xs[e] - m;
         }
-        __syncthreads();
-        const T m = (T)s_mean;
-        for (int e = threadIdx.x; e < n; e += blockDim.x) xa[e] = xr[e] - m;
         __syncthreads();
     }
-    // up: x' = x0 + sp P x_c (scratch), x = x' + w (b - A x') / diag
+    // up: x' = x + sp P x_c (scratch), then nu damped-Jacobi sweeps into the level's x
     for (int k = S.n - 2; k >= 0; --k) {
         const MgBlock Bf = mg_block(S.lv[k], b), Bc = mg_block(S.lv[k + 1], b);
         const int nf = Bf.sx * Bf.sy * Bf.sz, nc = Bc.sx * Bc.sy * Bc.sz;
@@ -862,27 +1004,22 @@ __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T
         T* sx = sb + nf;
         const T* sc = sx + nf;
         const T* sxc = sm + s_off[k + 1] + nc;
+        const MgCell cell(Bf);
         for (int e = threadIdx.x; e < nf; e += blockDim.x) {
             int x, y, z;
-            mg_unflatten(Bf, e, x, y, z);
+            cell.at<D>(Bf, e, x, y, z);
             scr[e] = sx[e] + sp * sxc[(x >> Bc.shx) + Bc.sx * ((y >> Bc.shy) + Bc.sy * (z >> Bc.shz))];
         }
         __syncthreads();
-        mg_sub_sweep<T, D>(Bf, nf, sc, sb, scr, sx, w);
+        mg_sub_sweep<T, D>(Bf, nf, sc, sb, scr, nu == 2 ? scr2 : sx, w);
         __syncthreads();
-        if (nu == 2) {  // second post-smoothing sweep
-            mg_sub_sweep<T, D>(Bf, nf, sc, sb, sx, scr, w);
-            __syncthreads();
-            for (int e = threadIdx.x; e < nf; e += blockDim.x) sx[e] = scr[e];
+        if (nu == 2) {
+            mg_sub_sweep<T, D>(Bf, nf, sc, sb, scr2, sx, w);
             __syncthreads();
         }
     }
-    {
-        const MgBlock B = mg_block(S.lv[0], b);
-        const int n = B.sx * B.sy * B.sz;
-        const T* sx = sm + s_off[0] + n;
-        for (int e = threadIdx.x; e < n; e += blockDim.x) xout[B.off + e] = sx[e];
-    }
+    const T* sx = sm + s_off[0] + n0;
+    for (int e = threadIdx.x; e < n0; e += blockDim.x) xout[B0.off + e] = sx[e];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -970,7 +1107,6 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom,
                                                               const double* __restrict__ sc, int first,
                                                               double* __restrict__ part, int cap_h, int cap_t,
                                                               int* __restrict__ err, const T* __restrict__ r) {
-    mg_pdl_entry();
     constexpr int K = 5;
     extern __shared__ __align__(128) unsigned char mg_bulk_raw[];
     __shared__ __align__(8) uint64_t bar[2];
@@ -987,18 +1123,30 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom,
     // this CTA's tiles blockIdx.x + j gridDim.x and their blocks, loaded once (the host guarantees at most
     // MG_BULK_MAX_TILES per CTA)
     const int all_tiles = (int)blockIdx.x < nt ? (nt - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    if (threadIdx.x == 0) {  // the live tiles, in order (tiles of converged systems are skipped)
-        int n = 0;
-        for (int j = 0; j < all_tiles; ++j) {
-            const int t = blockIdx.x + j * gridDim.x;
-            const MgTile tl = mg_tile(dom.tiles, t);
-            if (mg_done(sc, tl.sys)) continue;
-            s_tl[n] = tl;
-            s_bk[n] = mg_block(L, tl.blk);
-            s_tix[n] = t;
-            ++n;
+    static_assert(MG_BULK_MAX_TILES <= 64, "two warps list the tiles");
+    __shared__ int s_half;
+    {   // the live tiles, in order (tiles of converged systems are skipped): thread j reads tile j before the wait
+        const int j = threadIdx.x, lane = j & 31;
+        const bool mine = j < all_tiles;
+        MgTile tl = {};
+        MgBlock bk = {};
+        if (mine) {
+            tl = mg_tile(dom.tiles, blockIdx.x + j * gridDim.x);
+            bk = mg_block(L, tl.blk);
         }
-        s_nlive = n;
+        mg_pdl_wait();
+        mg_pdl_next();
+        const bool live = mine && !mg_done(sc, tl.sys);
+        const unsigned m = __ballot_sync(0xffffffffu, live);
+        if (j == 0) s_half = __popc(m);
+        __syncthreads();
+        if (j == 32) s_nlive = s_half + __popc(m);
+        if (live) {
+            const int n = (j < 32 ? 0 : s_half) + __popc(m & ((1u << lane) - 1u));
+            s_tl[n] = tl;
+            s_bk[n] = bk;
+            s_tix[n] = blockIdx.x + j * gridDim.x;
+        }
     }
 
     struct Runs {
@@ -1183,10 +1331,13 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_dot4(pict_domain_t dom, const T*
 template <int STRIDE>
 __global__ void k_pcg_scalars(pict_domain_t dom, const double* __restrict__ part, int stage, double* sc, int it,
                               double tol, int normalized, const int* __restrict__ ctr) {
-    mg_pdl_entry();
-    if (ctr) it += *ctr;
     const int lane = threadIdx.x & 31;
     const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int t0 = s < dom.num_sims ? dom.sim_tiles[s] * MG_NW : 0, t1 = s < dom.num_sims ? dom.sim_tiles[s + 1] * MG_NW : 0;
+    const int n = s < dom.num_sims ? dom.sim_cells[s + 1] - dom.sim_cells[s] : 1;
+    mg_pdl_wait();
+    mg_pdl_next();
+    if (ctr) it += *ctr;
     if (s >= dom.num_sims) return;
     if (stage != 0 && sc[MG_SC * s + 5] != 0.0) {  // converged earlier: keep its scalars
         if (stage == 2 && lane == 0) sc[MG_SC * s + 6] = 0.0;  // its last update has been applied
@@ -1196,8 +1347,7 @@ __global__ void k_pcg_scalars(pict_domain_t dom, const double* __restrict__ part
 #pragma unroll
     for (int k = 0; k < STRIDE; ++k) u[k] = 0.0;
     // two interleaved accumulators per lane (independent loads in flight), combined in a fixed order
-    const int t1 = dom.sim_tiles[s + 1] * MG_NW;
-    int t = dom.sim_tiles[s] * MG_NW + lane;
+    int t = t0 + lane;
     for (; t + 32 < t1; t += 64) {
 #pragma unroll
         for (int k = 0; k < STRIDE; ++k) {
@@ -1217,7 +1367,6 @@ __global__ void k_pcg_scalars(pict_domain_t dom, const double* __restrict__ part
         for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     if (lane != 0) return;
     double* S = sc + MG_SC * s;
-    const int n = dom.sim_cells[s + 1] - dom.sim_cells[s];
     if (stage == 1) {
         // alpha from p.q; with STRIDE 3 also |r - alpha q|^2 = |r|^2 - 2 alpha r.q + alpha^2 q.q: a system that
         // meets the tolerance here is done after this iteration's update (its V-cycle is skipped)
@@ -1408,31 +1557,55 @@ static pict_status_t run_pcg_mg(const pict_domain_t* dom, const pict_mg_level_t*
                                              (int)sub_smem);
         if (e != cudaSuccess) return set_error(PICT_ERR_CUDA, "pcg_mg: sub-cycle shared memory");
     }
-    // shared-memory stages of the 2D restriction / prolongation: x or x0, b, diag
-    const int cap = D == 2 ? MG_STAGE : 0;
-    const size_t stage3 = D == 2 ? 3 * (size_t)MG_STAGE * sizeof(T) : 0;
-    if (D == 2) {
-        cudaError_t e = cudaFuncSetAttribute(k_mg_restrict<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)stage3);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_mg_restrict<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)stage3);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_mg_prolong<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)stage3);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_mg_prolong<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)stage3);
-        if (e != cudaSuccess) return set_error(PICT_ERR_CUDA, "pcg_mg: stage shared memory");
-    }
-
     // smoothing sweeps per level of the tile kernels: the level's own choice (every tile's stage holds the
     // halo rows of two sweeps) capped by the process-wide setting; level 0 also needs the domain's tiles to
-    // fit the four-array stage of the two-sweep prolongation.  The one-launch sub-cycle takes the setting.
+    // fit the stage of the two-sweep prolongation.  The one-launch sub-cycle takes the setting.
+    const int cap = D == 2 ? MG_STAGE : 0;
     int nu[16];
     for (int l = 0; l < nl; ++l) nu[l] = (D == 2 && g_mg_sweeps >= 2 && levels[l].sweeps >= 2) ? 2 : 1;
     if (nu[0] == 2 && dom->tile_cells + 6 * levels[0].max_block_sx > (3 * cap) / 4) nu[0] = 1;
     const int nu_sub = g_mg_sweeps >= 2 ? 2 : 1;
+    // shared-memory stages of the 2D restriction / prolongation.  One sweep: x0 (or x'), b, diag of MG_STAGE cells.  Two
+    // sweeps: what the level's tiles need at most, so that small blocks leave room for more CTAs on an SM: a coarse
+    // tile of at most MG_TILE cells has at most (4 MG_TILE + 8 sx) fine cells with two halo rows on each side (rows
+    // that it covers partly included), a tile of the level its own cells and six rows.
+    const size_t stage3 = D == 2 ? 3 * (size_t)MG_STAGE * sizeof(T) : 0;
+    int cap_r[16], cap_p[16];
+    size_t sm_r[16], sm_p[16];
+    bool staged_r[16], staged_p[16];
+    for (int l = 0; l < nl; ++l) {
+        const int sx = levels[l].max_block_sx, tile = l == 0 ? dom->tile_cells : MG_TILE;
+        cap_r[l] = 4 * MG_TILE + 8 * sx < MG_STAGE ? 4 * MG_TILE + 8 * sx : MG_STAGE;
+        cap_p[l] = tile + 6 * sx;
+        // the couplings too where a launch is about one wave of CTAs, whose latency counts; with several waves the
+        // kernels are bound by throughput and more CTAs on an SM hide more (256 cavities: finest prolongation 69 us
+        // staged, 48..55 not; 16 cavities: 8.3 us staged)
+        const int tr = l + 1 < nl ? levels[l + 1].num_tiles : 0, tp = l == 0 ? nt : levels[l].num_tiles;
+        staged_r[l] = tr <= MG2_WAVES * device_sm_count();
+        staged_p[l] = tp <= MG2_WAVES * device_sm_count();
+        sm_r[l] = (staged_r[l] ? 6 : 3) * (size_t)cap_r[l] * sizeof(T);
+        sm_p[l] = (staged_p[l] ? 7 : 4) * (size_t)cap_p[l] * sizeof(T);
+        if (nu[l] == 2 && (sm_r[l] > MG2_MAX_SMEM || sm_p[l] > MG2_MAX_SMEM)) nu[l] = 1;
+    }
+    if constexpr (D == 2) {
+        cudaError_t e = cudaSuccess;
+        auto allow = [&](auto* k, size_t bytes) {
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        };
+        allow(k_mg_restrict<T, D, true>, stage3);
+        allow(k_mg_restrict<T, D, false>, stage3);
+        allow(k_mg_prolong<T, D, true>, stage3);
+        allow(k_mg_prolong<T, D, false>, stage3);
+        allow(k_mg_restrict2<T, true, true>, MG2_MAX_SMEM);
+        allow(k_mg_restrict2<T, true, false>, MG2_MAX_SMEM);
+        allow(k_mg_restrict2<T, false, true>, MG2_MAX_SMEM);
+        allow(k_mg_restrict2<T, false, false>, MG2_MAX_SMEM);
+        allow(k_mg_prolong2<T, true, true>, MG2_MAX_SMEM);
+        allow(k_mg_prolong2<T, true, false>, MG2_MAX_SMEM);
+        allow(k_mg_prolong2<T, false, true>, MG2_MAX_SMEM);
+        allow(k_mg_prolong2<T, false, false>, MG2_MAX_SMEM);
+        if (e != cudaSuccess) return set_error(PICT_ERR_CUDA, "pcg_mg: stage shared memory");
+    }
 
     // z = M r_new (V-cycle) and the per-warp partials of r_new.z, |r_new|^2, sum(z), sum(r_new).  upd:
     // the finest restriction first forms r_new = r - alpha q (stored to rn) and x += alpha p.
@@ -1448,22 +1621,36 @@ static pict_status_t run_pcg_mg(const pict_domain_t* dom, const pict_mg_level_t*
         for (int l = 0; l < lc; ++l) {
             const pict_mg_level_t& F = levels[l];
             const pict_mg_level_t& C = levels[l + 1];
-            if (l == 0 && upd)
-                mg_launch(k_mg_restrict<T, D, true>, C.num_tiles, MG_TPB, stage3, st, F, C, r, q, rn, xout, p, sc, first,
-                                                                                lb[1], wj, cap, sc, nu[0]);
+            const bool u = l == 0 && upd;
+            const T* src = l == 0 ? r : lb[l];
+            if (D == 2 && nu[l] == 2)
+                mg_launch(staged_r[l] ? (u ? k_mg_restrict2<T, true, true> : k_mg_restrict2<T, false, true>)
+                                      : (u ? k_mg_restrict2<T, true, false> : k_mg_restrict2<T, false, false>),
+                          C.num_tiles, staged_r[l] ? Mg2<true>::threads : Mg2<false>::threads, sm_r[l], st, F, C, src, u ? q : nullptr, u ? rn : nullptr, u ? xout : nullptr, u ? p : nullptr, sc, first, lb[l + 1], wj,
+                          cap_r[l]);
             else
-                mg_launch(k_mg_restrict<T, D, false>, C.num_tiles, MG_TPB, stage3, st, 
-                    F, C, l == 0 ? r : lb[l], nullptr, nullptr, nullptr, nullptr, nullptr, 0, lb[l + 1], wj, cap, sc,
-                    nu[l]);
+                mg_launch(u ? k_mg_restrict<T, D, true> : k_mg_restrict<T, D, false>, C.num_tiles, MG_TPB, stage3, st, F, C, src,
+                          u ? q : nullptr, u ? rn : nullptr, u ? xout : nullptr, u ? p : nullptr, u ? sc : nullptr, first,
+                          lb[l + 1], wj, cap, sc);
         }
         // levels lc.. in one launch (one CTA per block)
         mg_launch(k_mg_subcycle<T, D>, levels[lc].num_blocks, MG_SUB_THREADS, sub_smem, st, sub, lb[lc], lx[lc], wj, sp,
                                                                                   coarse_sweeps, sc, nu_sub);
-        for (int l = lc - 1; l >= 1; --l)
-            mg_launch(k_mg_prolong<T, D, false>, levels[l].num_tiles, MG_TPB, stage3, st, 
-                levels[l], levels[l + 1], levels[l].tiles, lb[l], lx[l + 1], lx[l], sp, wj, nullptr, cap, sc, nu[l]);
-        mg_launch(k_mg_prolong<T, D, true>, nt, MG_TPB, stage3, st, levels[0], levels[1], dom->tiles, rnew, lx[1], z, sp, wj,
-                                                             part, cap, sc, nu[0]);
+        for (int l = lc - 1; l >= 0; --l) {
+            const bool dot = l == 0;
+            const int tiles = dot ? nt : levels[l].num_tiles;
+            const int32_t* tab = dot ? dom->tiles : levels[l].tiles;
+            if (D == 2 && nu[l] == 2)
+                mg_launch(staged_p[l] ? (dot ? k_mg_prolong2<T, true, true> : k_mg_prolong2<T, false, true>)
+                                      : (dot ? k_mg_prolong2<T, true, false> : k_mg_prolong2<T, false, false>),
+                          tiles, staged_p[l] ? Mg2<true>::threads : Mg2<false>::threads, sm_p[l], st, levels[l], levels[l + 1],
+                          tab, dot ? rnew : lb[l], lx[l + 1], dot ? z : lx[l], sp, wj, dot ? part : nullptr,
+                          cap_p[l], sc);
+            else
+                mg_launch(dot ? k_mg_prolong<T, D, true> : k_mg_prolong<T, D, false>, tiles, MG_TPB, stage3, st, levels[l],
+                          levels[l + 1], tab, dot ? rnew : lb[l], lx[l + 1], dot ? z : lx[l], sp, wj, dot ? part : nullptr,
+                          cap, sc);
+        }
         return check_launch("pcg_mg vcycle");
     };
 

@@ -187,7 +187,7 @@ class MGHierarchy:
         esz = 8 if self.dtype == torch.float64 else 4
         for l in range(1, self.num_levels):
             cells = [int(self.levels[k].max_block_cells) for k in range(l, self.num_levels)]
-            smem = esz * (cells[0] + (2 + self.K) * sum(cells))
+            smem = esz * (2 * cells[0] + (2 + self.K) * sum(cells))
             if cells[0] <= SUB_MAX_CELLS and smem <= SUB_MAX_SMEM:
                 return l
         return self.num_levels - 1
