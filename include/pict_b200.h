@@ -250,9 +250,10 @@ pict_status_t pict_solve(const pict_domain_t* dom, const void* coef, const void*
                          int64_t workspace_bytes, void* stream);
 
 /* Process-wide choice of the launch form of the single-reduction CG (variant 1; no counterpart in the
- * reference): 1 (default) solves each system with one thread-block cluster (16 CTAs, else 8) when a
+ * reference) and of BiCGStab: 1 (default) solves each system with one thread-block cluster (16 CTAs, else 8) when a
  * domain holds few systems (at most 8) of at most 262,144 cells, reducing the inner products through
- * distributed shared memory with one cluster barrier per iteration and no grid-wide barrier; 0 always
+ * distributed shared memory with no grid-wide barrier (systems of up to 65,536 cells FP32 or 32,768 FP64, BiCGStab 16,384
+ * to 32,768 by type and components, with every vector in registers; BiCGStab above that takes the grid); 0 always
  * uses the persistent grid; 2 uses clusters whenever they fit. */
 void pict_krylov_set_cluster_mode(int32_t mode);
 /* BiCGStab kernel (no counterpart in the reference): 0 (default) four grid barriers per iteration for every

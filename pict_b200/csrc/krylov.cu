@@ -1877,8 +1877,10 @@ __global__ void __launch_bounds__(KR_THREADS, 2) k_cg1_cluster(KArgs<T> a) {
 
 namespace pict {
 
-__global__ void k_init_info(pict_solve_info_t* info, int n) {
+// reports of the right-hand sides c0 .. nrhs - 1 of every system
+__global__ void k_init_info(pict_solve_info_t* info, int n, int nrhs, int c0) {
     PICT_CELL_LOOP(i, n) {
+        if (i % nrhs < c0) continue;
         info[i].final_residual = 0.0;
         info[i].used_iterations = -1;
         info[i].converged = 0;
@@ -2023,21 +2025,26 @@ static pict_status_t launch_resident(void (*kern)(KArgs<T>, bool), size_t smem, 
     return PICT_OK;
 }
 
-template <typename T, int D, int CPT, bool ROWS_SMEM>
+template <typename T, int D, int CPT, bool ROWS_SMEM, bool COPIES>
 static pict_status_t launch_cg1_resident_as(KArgs<T>& a, bool trans, cudaStream_t st) {
-    return launch_resident<T>(k_cg1_resident<T, D, CPT, ROWS_SMEM>, resident_smem<T, D, CPT, ROWS_SMEM>(1), a, trans, st);
+    return launch_resident<T>(k_cg1_resident<T, D, CPT, ROWS_SMEM, COPIES>,
+                              resident_smem<T, D, CPT, ROWS_SMEM>(COPIES ? 2 : 1), a, trans, st);
 }
 
-// The stencil rows stay in registers while a thread's share fits 128 of them: up to 4 FP32 cells, 1 FP64 cell (2 in
-// 2D).  Beyond that they go to shared memory, up to 8 FP32 / 4 FP64 cells (65,536 / 32,768 cells a system).
+// What a thread's 128 registers hold decides the form: the neighbours' copies (one barrier an iteration) while they
+// fit, with the stencil rows in shared memory where only that makes room: 64^2 cells in FP32 205 -> 151 us a solve, 128^2
+// in FP64 the whole gradient 7.2 -> 6.8 ms.  From 4 cells a thread on two barriers are faster (27,648 cells: 6.44 ms a
+// pass, 6.68 with the copies and the rows in shared memory), with the rows in shared memory where registers end, up to
+// 8 FP32 / 4 FP64 cells a thread (65,536 / 32,768 cells a system).
 template <typename T, int D>
 static pict_status_t launch_cg1_resident(KArgs<T>& a, bool trans, cudaStream_t st) {
+    constexpr bool F64 = sizeof(T) == 8;
     const int cpt = resident_cpt(&a.dom);
-    if (cpt <= 1) return launch_cg1_resident_as<T, D, 1, false>(a, trans, st);
-    if (cpt <= 2) return launch_cg1_resident_as<T, D, 2, sizeof(T) == 8 && D == 3>(a, trans, st);
-    if (cpt <= 4) return launch_cg1_resident_as<T, D, 4, sizeof(T) == 8>(a, trans, st);
-    if constexpr (sizeof(T) == 4)
-        if (cpt <= 8) return launch_cg1_resident_as<T, D, 8, true>(a, trans, st);
+    if (cpt <= 1) return launch_cg1_resident_as<T, D, 1, false, true>(a, trans, st);
+    if (cpt <= 2) return launch_cg1_resident_as<T, D, 2, F64 || D == 3, !(F64 && D == 3)>(a, trans, st);
+    if (cpt <= 4) return launch_cg1_resident_as<T, D, 4, F64, false>(a, trans, st);
+    if constexpr (!F64)
+        if (cpt <= 8) return launch_cg1_resident_as<T, D, 8, true, false>(a, trans, st);
     return PICT_ERR_UNSUPPORTED;
 }
 
@@ -2106,14 +2113,12 @@ static pict_status_t run_solve(const pict_domain_t* dom, const void* coef, const
     const int nrhs_total = prm->nrhs;
     pict_solve_info_t* info = reinterpret_cast<pict_solve_info_t*>(info_out);
     const int ninfo = dom->num_sims * nrhs_total;
-    k_init_info<<<cell_grid(ninfo, 128), 128, 0, st>>>(info, ninfo);
-    pict_status_t s = check_launch("init_info");
-    if (s) return s;
+    pict_status_t s = PICT_OK;
+    bool prepared = false;
     const size_t NS = (size_t)dom->num_cells;
     const int per = nrhs_per_launch(prm);
     for (int c0 = 0; c0 < nrhs_total; c0 += per) {
         const int nr = (nrhs_total - c0) < per ? (nrhs_total - c0) : per;
-        if (cudaMemsetAsync(ctrl, 0, 256, st) != cudaSuccess) return check_launch("workspace memset");
         KArgs<T> a;
         a.dom = *dom;
         a.coef = reinterpret_cast<const T*>(coef);
@@ -2136,30 +2141,36 @@ static pict_status_t run_solve(const pict_domain_t* dom, const void* coef, const
         a.r1 = nullptr;
         a.nrhs = nrhs_total;
         void (*kern)(KArgs<T>) = nullptr;
-        if (prm->use_bicg) {
-            a.r = vec[0]; a.rw = vec[1]; a.p0 = vec[2]; a.p1 = vec[3]; a.v0 = vec[4]; a.v1 = vec[5]; a.t = vec[6];
-            a.r1 = vec[7];  // null with the four-barrier kernel (7 vectors)
-            const bool few_small = dom->num_sims <= 8;
-            if (a.abs_crit == 0 && g_bicgstab_variant == 0 && (g_cluster_mode == 2 || (g_cluster_mode == 1 && few_small))) {
-                s = PICT_ERR_UNSUPPORTED;
+        // few systems that fit one cluster's registers and shared memory: one launch, whose sums and waits stay in the
+        // cluster.  With many systems the lockstep grid amortises its barriers over all of them.
+        const bool cg1 = !prm->use_bicg && prm->variant == 1 && a.reset == 0 && a.best == 0 && a.abs_crit == 0 && a.rankdef == 0;
+        if (g_cluster_mode == 2 || (g_cluster_mode == 1 && dom->num_sims <= 8)) {
+            s = PICT_ERR_UNSUPPORTED;
+            if (cg1) s = launch_cg1_resident<T, D>(a, TRANS, st);
+            else if (prm->use_bicg && a.abs_crit == 0 && g_bicgstab_variant == 0) {
                 if (nr == 1) s = launch_bicgstab_resident<T, D, 1>(a, TRANS, st);
                 else if (nr == 2) s = launch_bicgstab_resident<T, D, 2>(a, TRANS, st);
                 else if constexpr (D == 3) s = launch_bicgstab_resident<T, D, 3>(a, TRANS, st);
-                if (s == PICT_OK) {
-                    k_finish_info<<<1, 128, 0, st>>>(info, ninfo, ctrl);
-                    s = check_launch("finish_info");
-                    if (s) return s;
-                    continue;
-                }
-                if (s != PICT_ERR_UNSUPPORTED) return s;
             }
+            if (s == PICT_OK) continue;
+            if (s != PICT_ERR_UNSUPPORTED) return s;
+        }
+        if (!prepared) {
+            k_init_info<<<cell_grid(ninfo, 128), 128, 0, st>>>(info, ninfo, nrhs_total, c0);
+            if ((s = check_launch("init_info"))) return s;
+            prepared = true;
+        }
+        if (cudaMemsetAsync(ctrl, 0, 256, st) != cudaSuccess) return check_launch("workspace memset");
+        if (prm->use_bicg) {
+            a.r = vec[0]; a.rw = vec[1]; a.p0 = vec[2]; a.p1 = vec[3]; a.v0 = vec[4]; a.v1 = vec[5]; a.t = vec[6];
+            a.r1 = vec[7];  // null with the four-barrier kernel (7 vectors)
             if (g_bicgstab_variant == 1 && a.abs_crit == 0 && nr <= 2)
                 kern = nr == 1 ? k_bicgstab2<T, D, 1, TRANS, 1> : k_bicgstab2<T, D, 2, TRANS, 1>;
             else if (g_bicgstab_variant == 2 && a.abs_crit == 0 && nr <= 2)
                 kern = nr == 1 ? k_bicgstab2<T, D, 1, TRANS, 2> : k_bicgstab2<T, D, 2, TRANS, 2>;
             else
                 kern = nr == 1 ? k_bicgstab<T, D, 1, TRANS> : (nr == 2 ? k_bicgstab<T, D, 2, TRANS> : k_bicgstab<T, D, 3, TRANS>);
-        } else if (prm->variant == 1 && a.reset == 0 && a.best == 0 && a.abs_crit == 0 && a.rankdef == 0) {
+        } else if (cg1) {
             a.r = vec[0]; a.rw = vec[1]; a.p0 = vec[2]; a.p1 = vec[3]; a.v0 = vec[4]; a.v1 = vec[5]; a.t = vec[6];
             kern = k_cg1<T, D, TRANS>;
             // one thread-block cluster per system where systems are small enough for one cluster's SMs to
@@ -2168,8 +2179,7 @@ static pict_status_t run_solve(const pict_domain_t* dom, const void* coef, const
             // them while each cluster would pay its own per system
             const bool few_small = dom->num_sims <= 8 && dom->max_sim_cells <= 262144;
             if (g_cluster_mode == 2 || (g_cluster_mode == 1 && few_small)) {
-                s = launch_cg1_resident<T, D>(a, TRANS, st);
-                if (s == PICT_ERR_UNSUPPORTED) s = launch_cg1_cluster<T, D, TRANS>(a, 16, st);
+                s = launch_cg1_cluster<T, D, TRANS>(a, 16, st);
                 if (s == PICT_ERR_UNSUPPORTED) s = launch_cg1_cluster<T, D, TRANS>(a, 8, st);
                 if (s == PICT_OK) {
                     k_finish_info<<<1, 128, 0, st>>>(info, ninfo, ctrl);

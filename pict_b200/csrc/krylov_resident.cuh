@@ -8,12 +8,12 @@
 // (distributed shared memory; each thread keeps the cluster addresses of its cells' neighbours, so connected and
 // periodic faces cost nothing extra).  Global memory is read once at the start and written once at the end.
 //
-// What bounds it: the chain of an iteration (for CG two cluster barriers, one remote read, one FP64 reduction), not
-// bytes: nothing but the result leaves the SMs.  The sweeping forms (k_cg1_cluster, and k_bicgstab with four grid
+// What bounds it: the chain of an iteration (for CG one or two cluster barriers, one remote read, one FP64 reduction),
+// not bytes: nothing but the result leaves the SMs.  The sweeping forms (k_cg1_cluster, and k_bicgstab with four grid
 // barriers an iteration) send every vector through L2 between barriers: ~5.5 us a CG iteration on up to 32k cells,
-// here ~2 us.  Measured, both with otherwise the same step: 8 steps of a 64^2 cavity in FP32 6.1 -> 3.2 ms, 2 steps
+// here 1.7 us (4,096 cells) to 2.1 us.  Measured on whole passes: 8 steps of a 64^2 cavity in FP32 6.8 -> 2.8 ms, 2 steps
 // of the 27,648-cell street 19.2 -> 6.4 ms, 2 steps of a 32^3 cavity in FP64 5.8 -> 2.8 ms, forward and backward of
-// 4 steps on a 128^2 periodic box in FP64 15.9 -> 7.2 ms.
+// 4 steps on a 128^2 periodic box in FP64 16.1 -> 6.8 ms.
 #pragma once
 
 namespace pict {
@@ -57,13 +57,14 @@ __device__ __forceinline__ void cluster_barrier() {
 // warps' sums by the first warp, its result pushed into every CTA's table, one cluster barrier, and the CTAs' sums by
 // a butterfly in every warp (no second block barrier).  Sum e writes table e & 1: a CTA gets there only after the
 // barrier of sum e - 1, which every CTA reaches only after it has read table e - 2.
+// In two parts, up to and with the barrier and after it, so that a caller can start the remote reads that the barrier
+// made visible before it waits for the sums.
 template <int NV>
-__device__ __forceinline__ void resident_sum(ResidentRed& R, int CL, int rank, unsigned& epoch, double (&v)[NV]) {
+__device__ __forceinline__ void resident_sum_push(ResidentRed& R, int CL, int rank, unsigned epoch, double (&v)[NV]) {
     static_assert(NV <= RS_NV, "resident_sum: too many values");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, par = epoch & 1;
-    ++epoch;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     }
@@ -89,7 +90,11 @@ __device__ __forceinline__ void resident_sum(ResidentRed& R, int CL, int rank, u
         __syncwarp();
     }
     cluster_barrier();
-    const int r = lane & 15;
+}
+
+template <int NV>
+__device__ __forceinline__ void resident_sum_read(ResidentRed& R, int CL, unsigned epoch, double (&v)[NV]) {
+    const int r = threadIdx.x & 15, par = epoch & 1;
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] = r < CL ? R.part[par][r][k] : 0.0;
 #pragma unroll
@@ -98,6 +103,16 @@ __device__ __forceinline__ void resident_sum(ResidentRed& R, int CL, int rank, u
         for (int k = 0; k < NV; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
     }
 }
+
+template <int NV>
+__device__ __forceinline__ void resident_sum(ResidentRed& R, int CL, int rank, unsigned& epoch, double (&v)[NV]) {
+    resident_sum_push<NV>(R, CL, rank, epoch, v);
+    resident_sum_read<NV>(R, CL, epoch, v);
+    ++epoch;
+}
+
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // The cells of this thread: stencil rows (registers, or shared memory when ROWS_SMEM) and neighbour addresses.
 template <typename T, int D, int CPT, bool ROWS_SMEM>
@@ -178,30 +193,26 @@ constexpr size_t resident_smem(int nbuf) {
     return sizeof(T) * (size_t)CPT * RS_THREADS * (nbuf + (ROWS_SMEM ? 2 * D + 1 : 0));
 }
 
-// CG, single-reduction recurrence (k_cg1): the iterates, stopping rule and reports of k_cg1_cluster.
-template <typename T, int D, int CPT, bool ROWS_SMEM>
+// CG, single-reduction recurrence (k_cg1): the iterates, stopping rule and reports of k_cg1_cluster.  COPIES: every
+// thread also carries r and s of its cells' neighbours and advances them with the neighbours' w, so an iteration needs
+// one cluster barrier (w and the sums together) instead of two (r, then the sums), for 4 D more values per cell.
+template <typename T, int D, int CPT, bool ROWS_SMEM, bool COPIES>
 __global__ void __launch_bounds__(RS_THREADS, 1) k_cg1_resident(KArgs<T> a, bool trans) {
     extern __shared__ __align__(16) unsigned char rs_smem[];
     __shared__ ResidentRed R;
-    __shared__ int s_sys;
     const pict_domain_t& dom = a.dom;
     cgrp::cluster_group cl = cgrp::this_cluster();
     const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     T* buf = reinterpret_cast<T*>(rs_smem);
+    constexpr unsigned WS = sizeof(T) * CPT * RS_THREADS;  // byte distance of the second exchange buffer (COPIES)
     ResidentRows<T, D, CPT, ROWS_SMEM> A;
-    A.sm = buf + CPT * RS_THREADS;
+    A.sm = buf + (COPIES ? 2 : 1) * CPT * RS_THREADS;
     unsigned epoch = 0;
     cluster_barrier();  // every CTA runs before any distributed shared memory access
 
-    for (;;) {
-        if (rank == 0 && threadIdx.x == 0) {
-            const int sys = atomicAdd(a.ctrl + CTRL_SCHED, 1);
-            for (int r = 0; r < CL; ++r) *cl.map_shared_rank(&s_sys, r) = sys;
-        }
-        __syncwarp();
-        cluster_barrier();
-        const int sys = s_sys;
-        if (sys >= dom.num_sims) break;
+    // the systems of this cluster: a fixed share (they are ordered largest first), so a solve is one launch that needs
+    // no cleared counter and writes every report itself
+    for (int sys = blockIdx.x / CL; sys < dom.num_sims; sys += gridDim.x / CL) {
         const int c0 = dom.sim_cells[sys], n = dom.sim_cells[sys + 1] - c0;
         const int run = (n + CL - 1) / CL;
         const int first = min(c0 + rank * run, c0 + n), cnt = min(run, c0 + n - first);
@@ -229,15 +240,36 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_cg1_resident(KArgs<T> a, bool
 #pragma unroll
         for (int k = 0; k < CPT; ++k) buf[k * RS_THREADS + threadIdx.x] = r[k];
         cluster_barrier();
+        T rn[COPIES ? CPT : 1][2 * D], sn[COPIES ? CPT : 1][2 * D], wn[COPIES ? CPT : 1][2 * D];
 #pragma unroll
         for (int k = 0; k < CPT; ++k) {
-            w[k] = A.apply(k, r[k]);
+            if constexpr (COPIES) {  // the neighbours' r0, and w0 into the second buffer
+                w[k] = A.get(k, 0) * r[k];
+#pragma unroll
+                for (int f = 0; f < 2 * D; ++f) {
+                    cluster_load(A.nb[k][f], rn[k][f]);
+                    sn[k][f] = T(0);
+                    w[k] += A.get(k, f + 1) * rn[k][f];
+                }
+                buf[(CPT + k) * RS_THREADS + threadIdx.x] = w[k];
+            } else {
+                w[k] = A.apply(k, r[k]);
+            }
             acc[0] += (double)r[k] * (double)r[k];
             acc[1] += (double)w[k] * (double)r[k];
         }
         resident_sum<3>(R, CL, rank, epoch, acc);
+        if constexpr (COPIES) {
+#pragma unroll
+            for (int k = 0; k < CPT; ++k)
+#pragma unroll
+                for (int f = 0; f < 2 * D; ++f) cluster_load(A.nb[k][f] + WS, wn[k][f]);
+        }
         pict_solve_info_t inf = fresh_info();
-        double g = acc[0], alpha = acc[0] / acc[1], beta = 0.0;
+        // crit < tol is tested as g' < tol^2 (n), which keeps a root and a division out of the iteration's chain (at
+        // least the smallest positive number, so that a residual of exactly 0 stops the tiniest tolerance too)
+        double g = acc[0], alpha = acc[0] / acc[1], beta = 0.0, gn = acc[0];
+        const double stop = a.tol > 0.0 ? fmax(a.tol * a.tol * (a.normalized ? (double)n : 1.0), 4.9406564584124654e-324) : -1.0;
         bool active = true;
         if (acc[2] == 0.0) {
             inf.converged = 1;
@@ -248,40 +280,70 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_cg1_resident(KArgs<T> a, bool
         }
         for (int it = 0; active && it < a.maxit; ++it) {
             const T al = (T)alpha, bt = (T)beta;
-#pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                p[k] = r[k] + bt * p[k];
-                s[k] = w[k] + bt * s[k];
-                r[k] -= al * s[k];
-                buf[k * RS_THREADS + threadIdx.x] = r[k];
-            }
-            cluster_arrive();
             double d[2] = {0.0, 0.0};
+            if constexpr (COPIES) {
+                // this thread's copies of the neighbours' s and r advance as their owners advance them (the same
+                // operations on the same values), so only w travels, together with the sums
+                const unsigned to = (it & 1) ? WS : 0u;
 #pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                x[k] += al * p[k];
-                d[0] += (double)r[k] * (double)r[k];
-            }
-            cluster_wait();
+                for (int k = 0; k < CPT; ++k) {
+                    p[k] = fma_rn(bt, p[k], r[k]);
+                    s[k] = fma_rn(bt, s[k], w[k]);
+                    r[k] = fma_rn(-al, s[k], r[k]);
+                    T acc_w = A.get(k, 0) * r[k];
 #pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                w[k] = A.apply(k, r[k]);
-                d[1] += (double)w[k] * (double)r[k];
+                    for (int f = 0; f < 2 * D; ++f) {
+                        sn[k][f] = fma_rn(bt, sn[k][f], wn[k][f]);
+                        rn[k][f] = fma_rn(-al, sn[k][f], rn[k][f]);
+                        acc_w += A.get(k, f + 1) * rn[k][f];
+                    }
+                    w[k] = acc_w;
+                    buf[(to ? CPT * RS_THREADS : 0) + k * RS_THREADS + threadIdx.x] = w[k];
+                    d[0] += (double)r[k] * (double)r[k];
+                    d[1] += (double)w[k] * (double)r[k];
+                }
+                resident_sum_push<2>(R, CL, rank, epoch, d);
+#pragma unroll
+                for (int k = 0; k < CPT; ++k)
+#pragma unroll
+                    for (int f = 0; f < 2 * D; ++f) cluster_load(A.nb[k][f] + to, wn[k][f]);
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) x[k] = fma_rn(al, p[k], x[k]);
+                resident_sum_read<2>(R, CL, epoch, d);
+                ++epoch;
+            } else {
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) {
+                    p[k] = r[k] + bt * p[k];
+                    s[k] = w[k] + bt * s[k];
+                    r[k] -= al * s[k];
+                    buf[k * RS_THREADS + threadIdx.x] = r[k];
+                }
+                cluster_arrive();
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) {
+                    x[k] += al * p[k];
+                    d[0] += (double)r[k] * (double)r[k];
+                }
+                cluster_wait();
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) {
+                    w[k] = A.apply(k, r[k]);
+                    d[1] += (double)w[k] * (double)r[k];
+                }
+                resident_sum<2>(R, CL, rank, epoch, d);
             }
-            resident_sum<2>(R, CL, rank, epoch, d);
-            const double gn = d[0];
-            const double crit = conv_crit(gn, a.normalized, n);
+            gn = d[0];
             inf.used_iterations = it;
-            inf.final_residual = crit;
-            if (!isfinite(crit)) { inf.finite = 0; active = false; }
-            else if (crit < a.tol) { inf.converged = 1; active = false; }
+            if (!isfinite(gn)) { inf.finite = 0; active = false; }
+            else if (gn < stop) { inf.converged = 1; active = false; }
             else {
-                const double bnew = gn / g;
-                alpha = gn / (d[1] - bnew * gn / alpha);
-                beta = bnew;
+                beta = gn / g;
+                alpha = gn / (d[1] - beta * gn / alpha);
                 g = gn;
             }
         }
+        if (inf.used_iterations >= 0 && acc[2] != 0.0) inf.final_residual = conv_crit(gn, a.normalized, n);
         T mean = T(0);
         if (a.sub_mean) {
             double m[1] = {0.0};
@@ -304,7 +366,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_cg1_resident(KArgs<T> a, bool
         }
         if (rank == 0 && threadIdx.x == 0) a.info[sys] = inf;
         __syncwarp();
-        cluster_barrier();  // every CTA is done with s_sys, the buffers and the table of this system
+        cluster_barrier();  // every CTA is done with the buffers and the tables of this system
     }
 }
 
@@ -316,7 +378,6 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_bicgstab_resident(KArgs<T> a,
     static_assert(2 * NR <= RS_NV, "too many right-hand sides per launch");
     extern __shared__ __align__(16) unsigned char rs_smem[];
     __shared__ ResidentRed R;
-    __shared__ int s_sys;
     constexpr int RUN = CPT * RS_THREADS;
     constexpr unsigned XS = sizeof(T) * RUN;          // byte distance from X[c] to X[c + 1]
     constexpr unsigned QS = sizeof(T) * RUN * NR;     // byte distance from X[c] to Q[c]
@@ -331,15 +392,9 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_bicgstab_resident(KArgs<T> a,
     unsigned epoch = 0;
     cluster_barrier();  // every CTA runs before any distributed shared memory access
 
-    for (;;) {
-        if (rank == 0 && threadIdx.x == 0) {
-            const int sys = atomicAdd(a.ctrl + CTRL_SCHED, 1);
-            for (int r = 0; r < CL; ++r) *cl.map_shared_rank(&s_sys, r) = sys;
-        }
-        __syncwarp();
-        cluster_barrier();
-        const int sys = s_sys;
-        if (sys >= dom.num_sims) break;
+    // the systems of this cluster: a fixed share (they are ordered largest first), so a solve is one launch that needs
+    // no cleared counter and writes every report itself
+    for (int sys = blockIdx.x / CL; sys < dom.num_sims; sys += gridDim.x / CL) {
         const int c0 = dom.sim_cells[sys], n = dom.sim_cells[sys + 1] - c0;
         const int run = (n + CL - 1) / CL;
         const int first = min(c0 + rank * run, c0 + n), cnt = min(run, c0 + n - first);
@@ -508,7 +563,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_bicgstab_resident(KArgs<T> a,
             for (int c = 0; c < NR; ++c) a.info[sys * a.nrhs + c] = inf[c];
         }
         __syncwarp();
-        cluster_barrier();  // every CTA is done with s_sys, the buffers and the tables of this system
+        cluster_barrier();  // every CTA is done with the buffers and the tables of this system
     }
 }
 

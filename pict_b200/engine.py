@@ -331,7 +331,8 @@ class PISOStepper:
         """Kernels of this library launched per step: advection setup 1; per solve init-info, solver and
         finish-info 3; per corrector pressure setup 2 (matrix/RHS, divergence), correction 1, and the
         refinement sweeps when enabled; the copy of the initial guess of a warm-started advection solve 1;
-        the advective outflow update 1."""
+        the advective outflow update 1.  An upper bound on domains of at most 8 systems that are solved
+        cluster-resident (one kernel per solve instead of three)."""
         n = 1 + 3 + (1 if self.warm_start_advection else 0) + (3 if self.advection_increment else 0) + \
             (1 if self.outflow else 0)
         n += self.corrector_steps * (2 + (3 if self.pressure_first_solve else 0) + 1)
