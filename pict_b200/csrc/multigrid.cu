@@ -95,6 +95,15 @@ __device__ __forceinline__ void mg_pdl_entry() {
 __device__ __forceinline__ void mg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mg_pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A kernel of the loop runs while its predecessor still writes, so an operand that any of them writes (vectors,
+// partials, scalars, the loop counter) is read through a plain pointer, after the wait: declared __restrict__ and only
+// read, it would count as constant during the kernel, and its load could take the read-only path ahead of the wait.
+// Stencils, which no kernel of the loop writes, are read as constants, also between a kernel's stores.
+template <typename T>
+__device__ __forceinline__ T mg_coef(const T* p) {
+    return __ldg(p);
+}
+
 __device__ __forceinline__ MgBlock mg_block(const pict_mg_level_t& L, int b) {
     const int* t = L.blocks + MG_BT * b;
     return MgBlock{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10]};
@@ -240,8 +249,8 @@ __device__ __forceinline__ void mg_nbrs(const MgBlock& B, int x, int y, int z, M
 // right-hand side of the finest V-cycle at a cell: r, or r - alpha q when the PCG update is fused
 template <typename T, bool UPD>
 struct MgRhs {
-    const T* __restrict__ r;
-    const T* __restrict__ q;
+    const T* r;
+    const T* q;
     T al;
     __device__ __forceinline__ T operator()(int j) const { return UPD ? r[j] - al * q[j] : r[j]; }
 };
@@ -261,6 +270,52 @@ __device__ __forceinline__ double* mg_warp_part(double* part, int stride) {
     return part + ((size_t)blockIdx.x * MG_NW + (threadIdx.x >> 5)) * stride;
 }
 
+// The right-hand side of the stage cells [0, n) of a restriction tile, cell 0 the first of row ylo at global cell lo,
+// handed to `put`; UPD: stored to rn, and x += alpha p (x = alpha p when first), for the children of the tile's coarse
+// cells lc0 .. lc1.  A thread reads MG_AHEAD cells before it writes any.
+constexpr int MG_AHEAD = 4;
+
+template <typename T, bool UPD, int TPB, typename F>
+__device__ __forceinline__ void mg_stage_rhs(const MgRhs<T, UPD>& rhs, T* rn, T* x, const T* p, int first, const MgBlock& Bc,
+                                             int lo, int ylo, int sx, int n, int lc0, int lc1, F&& put) {
+    const int dq = TPB / sx, dr = TPB - dq * sx;
+    int yy = (int)threadIdx.x / sx, xx = (int)threadIdx.x - yy * sx;
+    yy += ylo;
+    for (int e0 = threadIdx.x; e0 < n; e0 += MG_AHEAD * TPB) {
+        T bv[MG_AHEAD], xv[MG_AHEAD];
+        bool own[MG_AHEAD];
+#pragma unroll
+        for (int u = 0; u < MG_AHEAD; ++u) {
+            const int e = e0 + u * TPB, i = lo + e;
+            own[u] = false;
+            if (e < n) {
+                bv[u] = rhs(i);
+                if (UPD) {
+                    const int par = (xx >> Bc.shx) + Bc.sx * (yy >> Bc.shy);
+                    own[u] = par >= lc0 && par <= lc1;
+                    if (own[u]) xv[u] = first ? rhs.al * p[i] : x[i] + rhs.al * p[i];
+                    xx += dr;
+                    yy += dq;
+                    if (xx >= sx) {
+                        xx -= sx;
+                        ++yy;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < MG_AHEAD; ++u) {
+            const int e = e0 + u * TPB;
+            if (e >= n) break;
+            if (UPD && own[u]) {
+                rn[lo + e] = bv[u];
+                x[lo + e] = xv[u];
+            }
+            put(e, bv[u]);
+        }
+    }
+}
+
 // b_c = R (b - A x0) over the children of each coarse cell, x0 the pre-smoothed iterate from zero (levels with one
 // smoothing sweep).  UPD (finest level): b = r - alpha q is formed on the fly and stored to rn, and x += alpha p
 // (x = alpha p when first) for the children.
@@ -270,11 +325,9 @@ __device__ __forceinline__ double* mg_warp_part(double* part, int stride) {
 // cell sums its children's residuals from there (a y-periodic wrap forms x0 of that neighbour from global).
 template <typename T, int D, bool UPD>
 __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pict_mg_level_t C,
-                                                           const T* __restrict__ r, const T* __restrict__ q,
-                                                           T* __restrict__ rn, T* __restrict__ x,
-                                                           const T* __restrict__ p, const double* __restrict__ sc,
-                                                           int first, T* __restrict__ bc, T w, int cap,
-                                                           const double* __restrict__ dn) {
+                                                           const T* r, const T* q, T* rn, T* x, const T* p,
+                                                           const double* sc, int first, T* bc, T w, int cap,
+                                                           const double* dn) {
     mg_pdl_entry();
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(C.tiles, blockIdx.x);
@@ -284,21 +337,35 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int Nf = F.num_cells;
     const T al = UPD ? (T)sc[MG_SC * tl.sys + 1] : T(0);
-    if (UPD && pend) {  // converged at this iteration: the update of the children, no restriction
-        for (int k = threadIdx.x; k < tl.cnt; k += MG_TPB) {
+    // the update of the children of coarse cells k0 .. k1 - 1 of the tile (a thread's share of them)
+    auto update = [&](int k0, int k1) {
+        for (int k = k0 + (int)threadIdx.x; k < min(k1, tl.cnt); k += MG_TPB) {
             int X, Y, Z;
             mg_unflatten(Bc, tl.s0 + k - Bc.off, X, Y, Z);
+            T rv[1 << D], xv[1 << D];
+            int at[1 << D];
 #pragma unroll
             for (int c = 0; c < (1 << D); ++c) {
                 const int dx = c & 1, dy = (c >> 1) & 1, dz = (c >> 2) & 1;
                 const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy, zs = (Z << Bc.shz) + dz;
+                at[c] = -1;
                 if ((dx && !Bc.shx) || (dy && !Bc.shy) || (dz && !Bc.shz) || xs >= Bf.sx || ys >= Bf.sy || zs >= Bf.sz)
                     continue;
                 const int i = Bf.off + xs + Bf.sx * (ys + Bf.sy * zs);
-                rn[i] = r[i] - al * q[i];
-                x[i] = first ? al * p[i] : x[i] + al * p[i];
+                at[c] = i;
+                rv[c] = r[i] - al * q[i];
+                xv[c] = first ? al * p[i] : x[i] + al * p[i];
+            }
+#pragma unroll
+            for (int c = 0; c < (1 << D); ++c) {
+                if (at[c] < 0) continue;
+                rn[at[c]] = rv[c];
+                x[at[c]] = xv[c];
             }
         }
+    };
+    if (UPD && pend) {  // converged at this iteration: the update, no restriction
+        update(0, tl.cnt);
         return;
     }
     const MgRhs<T, UPD> rhs{r, q, al};
@@ -315,33 +382,16 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
         T* s_d = s_b + cap;
         const int lo = Bf.off + ylo * sx, nh = (yhi - ylo + 1) * sx;
         const int lc0 = tl.s0 - Bc.off, lc1 = lc0 + tl.cnt - 1;
-        const int dq = MG_TPB / sx, dr = MG_TPB - dq * sx;
-        int yy = (int)threadIdx.x / sx, xx = (int)threadIdx.x - yy * sx;
-        yy += ylo;
-        for (int e = threadIdx.x; e < nh; e += MG_TPB) {
-            const int i = lo + e;
-            const T bi = rhs(i), di = cf[i];
+        mg_stage_rhs<T, UPD, MG_TPB>(rhs, rn, x, p, first, Bc, lo, ylo, sx, nh, lc0, lc1, [&](int e, T bi) {
+            const T di = mg_coef(cf + lo + e);
             s_x0[e] = mg_x0(di, bi, w);
             s_d[e] = di;
             s_b[e] = bi;
-            if (UPD) {
-                const int par = (xx >> Bc.shx) + Bc.sx * (yy >> Bc.shy);
-                if (par >= lc0 && par <= lc1) {
-                    rn[i] = bi;
-                    x[i] = first ? al * p[i] : x[i] + al * p[i];
-                }
-            }
-            xx += dr;
-            yy += dq;
-            if (xx >= sx) {
-                xx -= sx;
-                ++yy;
-            }
-        }
+        });
         __syncthreads();
         auto far = [&](int xq, int yq) -> T {
             const int j = Bf.off + xq + sx * yq;
-            return mg_x0(cf[j], rhs(j), w);
+            return mg_x0(mg_coef(cf + j), rhs(j), w);
         };
         const int dqc = MG_TPB / Bc.sx, drc = MG_TPB - dqc * Bc.sx;
         const int l = lc0 + (int)threadIdx.x;
@@ -361,10 +411,10 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
                 const T ym = ys > 0 ? s_x0[c - sx] : (Bf.py ? far(xs, Bf.sy - 1) : T(0));
                 const T yp = ys + 1 < Bf.sy ? s_x0[c + sx] : (Bf.py ? far(xs, 0) : T(0));
                 T ax = s_d[c] * xi;
-                ax += (xs > 0 || Bf.px) ? cf[(size_t)Nf + i] * xm : T(0);
-                ax += (xs + 1 < sx || Bf.px) ? cf[(size_t)2 * Nf + i] * xp : T(0);
-                ax += (ys > 0 || Bf.py) ? cf[(size_t)3 * Nf + i] * ym : T(0);
-                ax += (ys + 1 < Bf.sy || Bf.py) ? cf[(size_t)4 * Nf + i] * yp : T(0);
+                ax += (xs > 0 || Bf.px) ? mg_coef(cf + (size_t)Nf + i) * xm : T(0);
+                ax += (xs + 1 < sx || Bf.px) ? mg_coef(cf + (size_t)2 * Nf + i) * xp : T(0);
+                ax += (ys > 0 || Bf.py) ? mg_coef(cf + (size_t)3 * Nf + i) * ym : T(0);
+                ax += (ys + 1 < Bf.sy || Bf.py) ? mg_coef(cf + (size_t)4 * Nf + i) * yp : T(0);
                 acc += s_b[c] - ax;
             }
             bc[tl.s0 + k] = acc;
@@ -402,21 +452,18 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
                 MgNbrs<D> nb;
                 mg_nbrs<D>(Bf, xs, ys, zs, nb);
                 const T bi = rhs(i);
-                const T di = cf[i];
+                const T di = mg_coef(cf + i);
                 T ax = di * mg_x0(di, bi, w);
 #pragma unroll
                 for (int f = 0; f < 2 * D; ++f) {
-                    const T cj = cf[(size_t)(f + 1) * Nf + i];
-                    const T xj = mg_x0(cf[nb.j[f]], rhs(nb.j[f]), w);
+                    const T cj = mg_coef(cf + (size_t)(f + 1) * Nf + i);
+                    const T xj = mg_x0(mg_coef(cf + nb.j[f]), rhs(nb.j[f]), w);
                     ax += nb.ok[f] ? cj * xj : T(0);
-                }
-                if (UPD && valid && live) {
-                    rn[i] = bi;
-                    x[i] = first ? al * p[i] : x[i] + al * p[i];
                 }
                 acc[k] += valid ? bi - ax : T(0);
             }
         }
+        if (UPD) update(base, base + MG_PASS);
 #pragma unroll
         for (int k = 0; k < MG_CPT; ++k) {
             const int l = base + k * MG_TPB + (int)threadIdx.x;
@@ -434,9 +481,8 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
 // y-periodic wrap reaches outside the stage and forms x' of that neighbour from global memory.
 template <typename T, int D, bool DOT>
 __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pict_mg_level_t C, const int32_t* tiles,
-                                                          const T* __restrict__ bv, const T* __restrict__ ec,
-                                                          T* __restrict__ out, T s, T w, double* __restrict__ part,
-                                                          int cap, const double* __restrict__ dn) {
+                                                          const T* bv, const T* ec, T* out, T s, T w, double* part,
+                                                          int cap, const double* dn) {
     mg_pdl_entry();
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(tiles, blockIdx.x);
@@ -457,7 +503,7 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
         int y = l / sx, x = l - y * sx;
         for (int e = threadIdx.x; e < hi - lo; e += MG_TPB) {
             const int i = lo + e;
-            const T d = cf[i], b = bv[i];
+            const T d = mg_coef(cf + i), b = bv[i];
             s_x[e] = mg_x0(d, b, w) + s * ec[Bc.off + (x >> Bc.shx) + Bc.sx * (y >> Bc.shy)];
             s_b[e] = b;
             s_d[e] = d;
@@ -472,7 +518,7 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
         // x' of a neighbour across the y-periodic wrap (outside the stage)
         auto far = [&](int xq, int yq) -> T {
             const int j = Bf.off + xq + sx * yq;
-            return mg_x0(cf[j], bv[j], w) + s * ec[Bc.off + (xq >> Bc.shx) + Bc.sx * (yq >> Bc.shy)];
+            return mg_x0(mg_coef(cf + j), bv[j], w) + s * ec[Bc.off + (xq >> Bc.shx) + Bc.sx * (yq >> Bc.shy)];
         };
         l = tl.s0 - Bf.off + (int)threadIdx.x;
         y = l / sx;
@@ -486,10 +532,10 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
             const T ym = y > 0 ? s_x[c - sx] : (Bf.py ? far(x, Bf.sy - 1) : T(0));
             const T yp = y + 1 < Bf.sy ? s_x[c + sx] : (Bf.py ? far(x, 0) : T(0));
             T acc = di * xi;
-            acc += okm ? cf[(size_t)N + i] * xm : T(0);
-            acc += okp ? cf[(size_t)2 * N + i] * xp : T(0);
-            acc += (y > 0 || Bf.py) ? cf[(size_t)3 * N + i] * ym : T(0);
-            acc += (y + 1 < Bf.sy || Bf.py) ? cf[(size_t)4 * N + i] * yp : T(0);
+            acc += okm ? mg_coef(cf + (size_t)N + i) * xm : T(0);
+            acc += okp ? mg_coef(cf + (size_t)2 * N + i) * xp : T(0);
+            acc += (y > 0 || Bf.py) ? mg_coef(cf + (size_t)3 * N + i) * ym : T(0);
+            acc += (y + 1 < Bf.sy || Bf.py) ? mg_coef(cf + (size_t)4 * N + i) * yp : T(0);
             const T zi = xi + ((di != T(0)) ? mg_div(w * (bi - acc), di) : T(0));
             out[i] = zi;
             if (DOT) {
@@ -517,15 +563,15 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
                 mg_unflatten(Bf, i - Bf.off, x, y, z);
                 MgNbrs<D> nb;
                 mg_nbrs<D>(Bf, x, y, z, nb);
-                const T di = cf[i], bi = bv[i];
+                const T di = mg_coef(cf + i), bi = bv[i];
                 const T xi = mg_x0(di, bi, w) + s * ec[mg_coarse_index(Bc, x, y, z)];
                 T acc = di * xi;
 #pragma unroll
                 for (int f = 0; f < 2 * D; ++f) {
                     const int j = nb.j[f];
-                    const T cj = cf[(size_t)(f + 1) * N + i];
+                    const T cj = mg_coef(cf + (size_t)(f + 1) * N + i);
                     const T xj =
-                        mg_x0(cf[j], bv[j], w) + s * ec[mg_coarse_index(Bc, nb.c[f][0], nb.c[f][1], nb.c[f][2])];
+                        mg_x0(mg_coef(cf + j), bv[j], w) + s * ec[mg_coarse_index(Bc, nb.c[f][0], nb.c[f][1], nb.c[f][2])];
                     acc += nb.ok[f] ? cj * xj : T(0);
                 }
                 zv[k] = xi + ((di != T(0)) ? mg_div(w * (bi - acc), di) : T(0));
@@ -582,22 +628,23 @@ constexpr size_t MG2_MAX_SMEM = 192 * 1024;  // of one two-sweep CTA (FP64 stage
 
 // (A v) at stage cell c (column x of rows of sx, stage of nst cells).  The diagonal term is kept beside the others and
 // not folded into a (1 - w) v, so that what is left of a constant v cancels here and is not carried through the sweeps.
-template <typename T>
+template <typename T, bool STAGED>
 __device__ __forceinline__ T mg2_apply(const T* v, const T* d, const T* cx, const T* cy, int c, int x, int sx, int nst) {
+    auto at = [](const T* a) { return STAGED ? *a : mg_coef(a); };
     const int m = x > 0 ? c - 1 : c + sx - 1, p = x + 1 < sx ? c + 1 : c - sx + 1;
-    T acc = d[c] * v[c];
-    acc += cx[m] * v[m];
-    acc += cx[c] * v[p];
-    if (c >= sx) acc += cy[c - sx] * v[c - sx];
-    if (c + sx < nst) acc += cy[c] * v[c + sx];
+    T acc = at(d + c) * v[c];
+    acc += at(cx + m) * v[m];
+    acc += at(cx + c) * v[p];
+    if (c >= sx) acc += at(cy + c - sx) * v[c - sx];
+    if (c + sx < nst) acc += at(cy + c) * v[c + sx];
     return acc;
 }
 
 // one damped-Jacobi sweep there: v + r (b - A v) with r = w / diag
-template <typename T>
+template <typename T, bool STAGED>
 __device__ __forceinline__ T mg2_sweep(const T* v, const T* b, const T* r, const T* d, const T* cx, const T* cy, int c, int x,
                                        int sx, int nst) {
-    return v[c] + r[c] * (b[c] - mg2_apply(v, d, cx, cy, c, x, sx, nst));
+    return v[c] + r[c] * (b[c] - mg2_apply<T, STAGED>(v, d, cx, cy, c, x, sx, nst));
 }
 
 template <bool STAGED>
@@ -624,10 +671,9 @@ __device__ __forceinline__ void mg2_stage_stencil(const T* __restrict__ cf, int 
 // UPD as k_mg_restrict.  Stage: the children's rows and two halo rows on each side (three arrays of `cap` cells, three more
 // when STAGED).
 template <typename T, bool UPD, bool STAGED>
-__global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_restrict2(pict_mg_level_t F, pict_mg_level_t C, const T* __restrict__ r,
-                                                             const T* __restrict__ q, T* __restrict__ rn, T* __restrict__ x,
-                                                             const T* __restrict__ p, const double* __restrict__ sc, int first,
-                                                             T* __restrict__ bc, T w, int cap) {
+__global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_restrict2(
+    pict_mg_level_t F, pict_mg_level_t C, const T* r, const T* q, T* rn, T* x, const T* p, const double* sc, int first, T* bc,
+    T w, int cap) {
     constexpr int MG2_TPB = Mg2<STAGED>::threads;
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(C.tiles, blockIdx.x);
@@ -646,34 +692,14 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
     const T* s_d = STAGED ? s_r + cap : cf + lo;
     const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * Nf + lo;
     const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * Nf + lo;
-    const int dq = MG2_TPB / sx, dr = MG2_TPB - dq * sx;
-    const int y0 = (int)threadIdx.x / sx, x0 = (int)threadIdx.x - y0 * sx;
+    const int dr = MG2_TPB % sx, x0 = (int)threadIdx.x % sx;
     mg_pdl_wait();
     mg_pdl_next();
     const bool pend = UPD && mg_pending(sc, tl.sys);
     if (mg_done(sc, tl.sys) && !pend) return;
     const T al = UPD ? (T)sc[MG_SC * tl.sys + 1] : T(0);
-    {
-        int xx = x0, yy = y0 + ylo;
-        for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
-            const int i = lo + e;
-            const T bi = UPD ? r[i] - al * q[i] : r[i];
-            if (UPD) {
-                const int par = (xx >> Bc.shx) + Bc.sx * (yy >> Bc.shy);
-                if (par >= lc0 && par <= lc1) {
-                    rn[i] = bi;
-                    x[i] = first ? al * p[i] : x[i] + al * p[i];
-                }
-                xx += dr;
-                yy += dq;
-                if (xx >= sx) {
-                    xx -= sx;
-                    ++yy;
-                }
-            }
-            s_b[e] = bi;
-        }
-    }
+    mg_stage_rhs<T, UPD, MG2_TPB>(MgRhs<T, UPD>{r, q, al}, rn, x, p, first, Bc, lo, ylo, sx, nst, lc0, lc1,
+                                  [&](int e, T bi) { s_b[e] = bi; });
     if (pend) return;  // converged at this iteration: only the update of its cells
     __syncthreads();
     {   // x1 = x0 + w (b - A x0) / diag with x0 = (w / diag) b formed from the stage.  Cells of the outermost rows whose
@@ -702,7 +728,7 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
             const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy;
             if ((dx && !Bc.shx) || (dy && !Bc.shy) || xs >= sx || ys >= Bf.sy) continue;
             const int c = (ys - ylo) * sx + xs;
-            acc += s_b[c] - mg2_apply(s_x, s_d, s_cx, s_cy, c, xs, sx, nst);
+            acc += s_b[c] - mg2_apply<T, STAGED>(s_x, s_d, s_cx, s_cy, c, xs, sx, nst);
         }
         bc[tl.s0 + k] = acc;
     }
@@ -714,10 +740,9 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
 // three halo rows on each side (four arrays of
 // `cap` cells, three more when STAGED).
 template <typename T, bool DOT, bool STAGED>
-__global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_prolong2(pict_mg_level_t F, pict_mg_level_t C, const int32_t* tiles,
-                                                            const T* __restrict__ bv, const T* __restrict__ ec,
-                                                            T* __restrict__ out, T s, T w, double* __restrict__ part, int cap,
-                                                            const double* __restrict__ sc) {
+__global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_prolong2(
+    pict_mg_level_t F, pict_mg_level_t C, const int32_t* tiles, const T* bv, const T* ec, T* out, T s, T w, double* part,
+    int cap, const double* sc) {
     constexpr int MG2_TPB = Mg2<STAGED>::threads;
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     __shared__ double s_red[MG2_TPB / 32][4];
@@ -767,14 +792,14 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_pro
     };
     const int t0 = tl.s0 - lo, t1 = t0 + tl.cnt;
     cells(max(0, t0 - 2 * sx), min(nst, t1 + 2 * sx),
-          [&](int c, int x) { s_y[c] += mg2_sweep(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+          [&](int c, int x) { s_y[c] += mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
     __syncthreads();
     cells(max(0, t0 - sx), min(nst, t1 + sx),
-          [&](int c, int x) { s_x[c] = mg2_sweep(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+          [&](int c, int x) { s_x[c] = mg2_sweep<T, STAGED>(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
     __syncthreads();
     double a = 0.0, c2 = 0.0, sz = 0.0, sr = 0.0;
     cells(t0, t1, [&](int c, int x) {
-        const T zi = mg2_sweep(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst);
+        const T zi = mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst);
         out[lo + c] = zi;
         if (DOT) {
             const double bi = (double)s_b[c];
@@ -874,9 +899,8 @@ __device__ __forceinline__ void mg_sub_sweep(const MgBlock& B, int n, const T* s
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T* __restrict__ bin,
-                                                                T* __restrict__ xout, T w, T sp, int sweeps,
-                                                                const double* __restrict__ dn, int nu) {
+__global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T* bin, T* xout, T w, T sp,
+                                                                int sweeps, const double* dn, int nu) {
     constexpr int K = 2 * D + 1;
     extern __shared__ __align__(16) unsigned char mg_sub_raw[];
     T* sm = reinterpret_cast<T*>(mg_sub_raw);
@@ -1030,10 +1054,9 @@ __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T
 // p_old = z with beta = 0), q = A p_new, and the per-warp partials of p_new.q (one CTA per work tile of
 // the domain); m, beta per system from sc
 template <typename T, int D>
-__global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot(pict_domain_t dom, pict_mg_level_t L, const T* __restrict__ z,
-                                                         const T* __restrict__ pold, T* __restrict__ pnew,
-                                                         T* __restrict__ q, const double* __restrict__ sc, int first,
-                                                         double* __restrict__ part, const T* __restrict__ r) {
+__global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot(pict_domain_t dom, pict_mg_level_t L, const T* z,
+                                                         const T* pold, T* pnew, T* q, const double* sc, int first,
+                                                         double* part, const T* r) {
     mg_pdl_entry();
     const T* __restrict__ coef = reinterpret_cast<const T*>(L.coef);
     const int N = L.num_cells;
@@ -1044,7 +1067,7 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot(pict_domain_t dom, pict
     const T bt = first ? T(0) : (T)sc[MG_SC * tl.sys + 2];
     double acc = 0.0, arq = 0.0, aqq = 0.0;
     for (int base = 0; base < tl.cnt; base += MG_PASS) {
-        T pv[MG_CPT], qv[MG_CPT];
+        T pv[MG_CPT], qv[MG_CPT], rv[MG_CPT];
 #pragma unroll
         for (int k = 0; k < MG_CPT; ++k) {
             const int l0 = base + k * MG_TPB + (int)threadIdx.x;
@@ -1055,16 +1078,17 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot(pict_domain_t dom, pict
             MgNbrs<D> nb;
             mg_nbrs<D>(B, x, y, z3, nb);
             const T pi = (z[i] - m) + bt * pold[i];
-            T qi = coef[i] * pi;
+            T qi = mg_coef(coef + i) * pi;
 #pragma unroll
             for (int f = 0; f < 2 * D; ++f) {
                 const int j = nb.j[f];
-                const T cj = coef[(size_t)(f + 1) * N + i];
+                const T cj = mg_coef(coef + (size_t)(f + 1) * N + i);
                 const T pj = (z[j] - m) + bt * pold[j];
                 qi += nb.ok[f] ? cj * pj : T(0);
             }
             pv[k] = pi;
             qv[k] = qi;
+            rv[k] = r[i];
         }
 #pragma unroll
         for (int k = 0; k < MG_CPT; ++k) {
@@ -1074,7 +1098,7 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot(pict_domain_t dom, pict
             q[tl.s0 + l] = qv[k];
             const double qd = (double)qv[k];
             acc += (double)pv[k] * qd;
-            arq += (double)r[tl.s0 + l] * qd;
+            arq += (double)rv[k] * qd;
             aqq += qd * qd;
         }
     }
@@ -1102,11 +1126,9 @@ constexpr int MG_BULK_MAX_TILES = 64;  // tiles per CTA of the persistent grid (
 
 template <typename T>
 __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom, pict_mg_level_t L,
-                                                              const T* __restrict__ z, const T* __restrict__ pold,
-                                                              T* __restrict__ pnew, T* __restrict__ q,
-                                                              const double* __restrict__ sc, int first,
-                                                              double* __restrict__ part, int cap_h, int cap_t,
-                                                              int* __restrict__ err, const T* __restrict__ r) {
+                                                              const T* z, const T* pold, T* pnew, T* q, const double* sc,
+                                                              int first, double* part, int cap_h, int cap_t, int* err,
+                                                              const T* r) {
     constexpr int K = 5;
     extern __shared__ __align__(128) unsigned char mg_bulk_raw[];
     __shared__ __align__(8) uint64_t bar[2];
@@ -1219,7 +1241,7 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom,
         const T* const c4 = buf + 2 * cap_h + 4 * cap_t + R.c[4].lead;
         double acc = 0.0, arq = 0.0, aqq = 0.0;
         for (int base = 0; base < tl.cnt; base += MG_PASS) {
-            T pvk[MG_CPT], qvk[MG_CPT];
+            T pvk[MG_CPT], qvk[MG_CPT], rvk[MG_CPT];
 #pragma unroll
             for (int kk = 0; kk < MG_CPT; ++kk) {
                 const int l0 = base + kk * MG_TPB + (int)threadIdx.x;
@@ -1267,6 +1289,7 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom,
                 }
                 pvk[kk] = pi;
                 qvk[kk] = qi;
+                rvk[kk] = r[i];
             }
 #pragma unroll
             for (int kk = 0; kk < MG_CPT; ++kk) {
@@ -1276,7 +1299,7 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom,
                 q[tl.s0 + l] = qvk[kk];
                 const double qd = (double)qvk[kk];
                 acc += (double)pvk[kk] * qd;
-                arq += (double)r[tl.s0 + l] * qd;
+                arq += (double)rvk[kk] * qd;
                 aqq += qd * qd;
             }
         }
@@ -1296,7 +1319,7 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_spmv_dot_bulk(pict_domain_t dom,
 // per-warp partials of r.z, r.r, sum(z), sum(r) (one CTA per work tile)
 template <typename T>
 __global__ void __launch_bounds__(MG_TPB) k_pcg_dot4(pict_domain_t dom, const T* r, const T* z, double* part,
-                                                     const double* __restrict__ dn) {
+                                                     const double* dn) {
     mg_pdl_entry();
     const MgTile tl = mg_tile(dom.tiles, blockIdx.x);
     if (mg_done(dn, tl.sys)) return;
@@ -1329,8 +1352,8 @@ __global__ void __launch_bounds__(MG_TPB) k_pcg_dot4(pict_domain_t dom, const T*
 // undetermined.  sc[s*MG_SC + {0: rho, 1: alpha, 2: beta, 3: |r|^2, 4: m}]
 // it: the PCG iteration; inside a graph's conditional loop it is an offset to the device counter ctr
 template <int STRIDE>
-__global__ void k_pcg_scalars(pict_domain_t dom, const double* __restrict__ part, int stage, double* sc, int it,
-                              double tol, int normalized, const int* __restrict__ ctr) {
+__global__ void k_pcg_scalars(pict_domain_t dom, const double* part, int stage, double* sc, int it, double tol, int normalized,
+                              const int* ctr) {
     const int lane = threadIdx.x & 31;
     const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int t0 = s < dom.num_sims ? dom.sim_tiles[s] * MG_NW : 0, t1 = s < dom.num_sims ? dom.sim_tiles[s + 1] * MG_NW : 0;
@@ -1403,10 +1426,8 @@ __global__ void k_pcg_scalars(pict_domain_t dom, const double* __restrict__ part
 // (0, rn.rn, 0, sum(rn)) (the PCG update where no V-cycle follows: the last iteration, or a
 // single-level hierarchy)
 template <typename T>
-__global__ void __launch_bounds__(MG_TPB) k_pcg_update(pict_domain_t dom, const T* __restrict__ r,
-                                                       const T* __restrict__ q, T* __restrict__ rn, T* __restrict__ x,
-                                                       const T* __restrict__ p, const double* __restrict__ sc, int first,
-                                                       double* __restrict__ part) {
+__global__ void __launch_bounds__(MG_TPB) k_pcg_update(pict_domain_t dom, const T* r, const T* q, T* rn, T* x,
+                                                       const T* p, const double* sc, int first, double* part) {
     mg_pdl_entry();
     const MgTile tl = mg_tile(dom.tiles, blockIdx.x);
     if (mg_done(sc, tl.sys) && !mg_pending(sc, tl.sys)) return;
@@ -1454,8 +1475,8 @@ __global__ void k_pcg_report(pict_domain_t dom, const double* sc, pict_solve_inf
 
 // Condition of the graph's PCG loop (one CTA): ctr = init (init > 0) or ctr += step, then keep looping
 // while a system is still iterating and the next two iterations (ctr, ctr + 1) are within the cap.
-__global__ void k_pcg_loop_cond(pict_domain_t dom, const double* __restrict__ sc, int* ctr, int init, int step,
-                                int limit, cudaGraphConditionalHandle h) {
+__global__ void k_pcg_loop_cond(pict_domain_t dom, const double* sc, int* ctr, int init, int step, int limit,
+                                cudaGraphConditionalHandle h) {
     mg_pdl_entry();
     __shared__ int s_any;
     if (threadIdx.x == 0) s_any = 0;
