@@ -208,6 +208,16 @@ __device__ __forceinline__ T mg_x0(T d, T b, T w) {
     return (d != T(0)) ? mg_div(w * b, d) : T(0);
 }
 
+// Relaxation weight in a block: 0 in a block of one cell.  Its operator, the sum of all couplings of the system, is 0 up
+// to rounding (the constant mode is singular), so a sweep there would divide by noise and add a constant many orders
+// above the solution, which the finer levels cancel only to their rounding: a 32^2 cavity beside one of 256^2 (its
+// block has one cell on the last two of seven levels) stalled at 1e-5 to 1e-4 of its right-hand side instead of 1e-8.
+// The coarsest level removes the mean anyway.
+template <typename T>
+__device__ __forceinline__ T mg_weight(const MgBlock& B, T w) {
+    return B.sx * B.sy * B.sz == 1 ? T(0) : w;
+}
+
 // The neighbours of a cell across its 2D faces, branch-free: where a fixed face has no neighbour the
 // index is the cell itself and ok is false (its term is masked), so every gather load is unconditional
 // and the loads of several cells can be in flight together.
@@ -334,6 +344,7 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_restrict(pict_mg_level_t F, pi
     const bool pend = UPD && mg_pending(sc, tl.sys);
     if (mg_done(dn, tl.sys) && !pend) return;
     const MgBlock Bc = mg_block(C, tl.blk), Bf = mg_block(F, tl.blk);
+    w = mg_weight(Bf, w);
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int Nf = F.num_cells;
     const T al = UPD ? (T)sc[MG_SC * tl.sys + 1] : T(0);
@@ -488,6 +499,7 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
     const MgTile tl = mg_tile(tiles, blockIdx.x);
     if (mg_done(dn, tl.sys)) return;
     const MgBlock Bf = mg_block(F, tl.blk), Bc = mg_block(C, tl.blk);
+    w = mg_weight(Bf, w);
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int N = F.num_cells;
     double a = 0.0, c2 = 0.0, sz = 0.0, sr = 0.0;
@@ -678,6 +690,7 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(C.tiles, blockIdx.x);
     const MgBlock Bc = mg_block(C, tl.blk), Bf = mg_block(F, tl.blk);
+    w = mg_weight(Bf, w);
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int Nf = F.num_cells, sx = Bf.sx;
     const int lc0 = tl.s0 - Bc.off, lc1 = lc0 + tl.cnt - 1;
@@ -748,6 +761,7 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_pro
     __shared__ double s_red[MG2_TPB / 32][4];
     const MgTile tl = mg_tile(tiles, blockIdx.x);
     const MgBlock Bf = mg_block(F, tl.blk), Bc = mg_block(C, tl.blk);
+    w = mg_weight(Bf, w);
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int N = F.num_cells, sx = Bf.sx, nf = sx * Bf.sy;
     const int lo = max(Bf.off, tl.s0 - 3 * sx), hi = min(Bf.off + nf, tl.s0 + tl.cnt + 3 * sx), nst = hi - lo;
@@ -888,6 +902,7 @@ __device__ __forceinline__ T mg_sub_off(const MgBlock& B, int n, const T* sc, co
 template <typename T, int D>
 __device__ __forceinline__ void mg_sub_sweep(const MgBlock& B, int n, const T* sc, const T* sb, const T* xs, T* xd,
                                              T w) {
+    w = mg_weight(B, w);
     const MgCell cell(B);
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         int x, y, z;
@@ -945,7 +960,7 @@ __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T
         const T* sc = sx + nf;
         T* sbc = sm + s_off[k + 1];
         T* x0 = nu == 2 ? scr : sx;
-        for (int e = threadIdx.x; e < nf; e += blockDim.x) x0[e] = mg_x0(sc[e], sb[e], w);
+        for (int e = threadIdx.x; e < nf; e += blockDim.x) x0[e] = mg_x0(sc[e], sb[e], mg_weight(Bf, w));
         __syncthreads();
         if (nu == 2) {
             mg_sub_sweep<T, D>(Bf, nf, sc, sb, scr, sx, w);
@@ -979,18 +994,19 @@ __global__ void __launch_bounds__(MG_SUB_THREADS) k_mg_subcycle(MgSub S, const T
         const T* sc = xa + n;
         if (n <= 32) {
             if (threadIdx.x < 32) {
+                const T wb = mg_weight(B, w);
                 const int e = threadIdx.x;
                 const bool in = e < n;
                 int x = 0, y = 0, z = 0;
                 if (in) MgCell(B).at<D>(B, e, x, y, z);
                 const T d = in ? sc[e] : T(0), be = in ? sb[e] : T(0);
-                T v = mg_x0(d, be, w);
+                T v = mg_x0(d, be, wb);
                 for (int it = 1; it < sweeps; ++it) {
                     if (in) xa[e] = v;
                     __syncwarp();
                     const T off = in ? mg_sub_off<T, D>(B, n, sc, xa, e, x, y, z) : T(0);
                     __syncwarp();
-                    v += (d != T(0)) ? mg_div(w * (be - (d * v + off)), d) : T(0);
+                    v += (d != T(0)) ? mg_div(wb * (be - (d * v + off)), d) : T(0);
                 }
                 const double m = mg_warp_sum(in ? (double)v : 0.0) / (double)n;
                 if (in) xa[e] = v - (T)m;
