@@ -322,7 +322,10 @@ typedef struct pict_mg_level {
     int32_t max_block_sx;      /* largest x size (cells per row) of a block of the level */
     int32_t sweeps;            /* damped-Jacobi sweeps of each smoothing step at this level when the restriction
                                   and prolongation tile kernels handle it: 2 where every tile's shared-memory
-                                  stage holds two halo rows (2D, not y-periodic), else 1 (0 reads as 1) */
+                                  stage holds two halo rows (2D, not y-periodic), else 1 (0 reads as 1).  The
+                                  tiles may have any size, larger ones than the stages are walked in runs that fit;
+                                  levels with rows of 512 cells or more, or with max_block_sx 0, are smoothed
+                                  once.  A block wider than max_block_sx is reported: status 1, not converged */
 } pict_mg_level_t;
 
 /* Process-wide choice of the 2D PCG SpMV kernel (no counterpart in the reference): 1 (default) stages

@@ -634,9 +634,9 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
 // ---------------------------------------------------------------------------------------------
 // STAGED keeps the couplings in shared memory too (512 threads, two CTAs on an SM); otherwise they are read through L1
 // where they are used (256 threads, more CTAs on an SM).
-constexpr int MG_TILE = 512;                  // cells of a coarse level's work tile (multigrid.py TILE_CELLS)
 constexpr int MG2_WAVES = 4;                  // CTAs per SM up to which a launch counts as one wave
 constexpr size_t MG2_MAX_SMEM = 192 * 1024;  // of one two-sweep CTA (FP64 stages of the widest blocks)
+constexpr int MG_TILE = 512;  // cells of a tile that the stages hold whole (the work tiles of the framework's coarse levels)
 
 // (A v) at stage cell c (column x of rows of sx, stage of nst cells).  The diagonal term is kept beside the others and
 // not folded into a (1 - w) v, so that what is left of a constant v cancels here and is not carried through the sweeps.
@@ -681,11 +681,11 @@ __device__ __forceinline__ void mg2_stage_stencil(const T* __restrict__ cf, int 
 
 // b_c = R (b - A x1) over the children of each coarse cell, x1 the pre-smoothed iterate after two sweeps from zero.
 // UPD as k_mg_restrict.  Stage: the children's rows and two halo rows on each side (three arrays of `cap` cells, three more
-// when STAGED).
+// when STAGED), which hold the framework's tiles whole; a larger tile is walked in runs that fit.
 template <typename T, bool UPD, bool STAGED>
 __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_restrict2(
     pict_mg_level_t F, pict_mg_level_t C, const T* r, const T* q, T* rn, T* x, const T* p, const double* sc, int first, T* bc,
-    T w, int cap) {
+    T w, int cap, int* err) {
     constexpr int MG2_TPB = Mg2<STAGED>::threads;
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     const MgTile tl = mg_tile(C.tiles, blockIdx.x);
@@ -693,69 +693,96 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
     w = mg_weight(Bf, w);
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int Nf = F.num_cells, sx = Bf.sx;
-    const int lc0 = tl.s0 - Bc.off, lc1 = lc0 + tl.cnt - 1;
-    const int ylo = max(0, ((lc0 / Bc.sx) << Bc.shy) - 2);
-    const int yhi = min(Bf.sy - 1, ((lc1 / Bc.sx + 1) << Bc.shy) + 1);
-    const int lo = Bf.off + ylo * sx, nst = (yhi - ylo + 1) * sx;
-    if (nst > cap) return;  // a tile table that does not keep the level's promise (sweeps = 2) stays in bounds
+    // the coarse cells [c0, c1) of the tile at a time, with fine rows from ylo on (nst cells): the whole tile, or as many
+    // coarse rows as fit the stage
+    const int cend = tl.s0 - Bc.off + tl.cnt;
+    int c0 = tl.s0 - Bc.off, c1, ylo, nst;
+    auto rows = [&] {
+        ylo = max(0, ((c0 / Bc.sx) << Bc.shy) - 2);
+        nst = (min(Bf.sy - 1, (((c1 - 1) / Bc.sx + 1) << Bc.shy) + 1) - ylo + 1) * sx;
+    };
+    auto fit = [&] {
+        c1 = cend;
+        rows();
+        if (nst > cap) {
+            c1 = min(cend, (c0 / Bc.sx + max((cap / sx - 4) >> Bc.shy, 1)) * Bc.sx);
+            rows();
+        }
+    };
+    fit();
     T* s_x = reinterpret_cast<T*>(mg_stage_raw);  // x1
     T* s_b = s_x + cap;
     T* s_r = s_b + cap;
-    mg2_stage_stencil<T, STAGED>(cf, Nf, lo, nst, w, s_r, s_r + cap, s_r + 2 * cap, s_r + 3 * cap);
-    const T* s_d = STAGED ? s_r + cap : cf + lo;
-    const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * Nf + lo;
-    const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * Nf + lo;
+    auto stage = [&] {
+        if (nst <= cap) mg2_stage_stencil<T, STAGED>(cf, Nf, Bf.off + ylo * sx, nst, w, s_r, s_r + cap, s_r + 2 * cap, s_r + 3 * cap);
+    };
+    stage();
     const int dr = MG2_TPB % sx, x0 = (int)threadIdx.x % sx;
     mg_pdl_wait();
     mg_pdl_next();
     const bool pend = UPD && mg_pending(sc, tl.sys);
     if (mg_done(sc, tl.sys) && !pend) return;
     const T al = UPD ? (T)sc[MG_SC * tl.sys + 1] : T(0);
-    mg_stage_rhs<T, UPD, MG2_TPB>(MgRhs<T, UPD>{r, q, al}, rn, x, p, first, Bc, lo, ylo, sx, nst, lc0, lc1,
-                                  [&](int e, T bi) { s_b[e] = bi; });
-    if (pend) return;  // converged at this iteration: only the update of its cells
-    __syncthreads();
-    {   // x1 = x0 + w (b - A x0) / diag with x0 = (w / diag) b formed from the stage.  Cells of the outermost rows whose
-        // outer neighbour row is outside the stage get a value that no child reads.
-        int xx = x0;
-        for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
-            const int m = xx > 0 ? e - 1 : e + sx - 1, pp = xx + 1 < sx ? e + 1 : e - sx + 1;
-            const T rc = s_r[e], xi = rc * s_b[e];
-            T acc = s_d[e] * xi;
-            acc += s_cx[m] * (s_r[m] * s_b[m]);
-            acc += s_cx[e] * (s_r[pp] * s_b[pp]);
-            if (e >= sx) acc += s_cy[e - sx] * (s_r[e - sx] * s_b[e - sx]);
-            if (e + sx < nst) acc += s_cy[e] * (s_r[e + sx] * s_b[e + sx]);
-            s_x[e] = xi + rc * (s_b[e] - acc);
-            xx += dr;
-            if (xx >= sx) xx -= sx;
+    for (;;) {
+        if (nst > cap) {  // a block wider than the level announced
+            if (threadIdx.x == 0) *err = 1;
+            return;
         }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < tl.cnt; k += MG2_TPB) {
-        const int l = lc0 + k, Y = l / Bc.sx, X = l - Y * Bc.sx;
-        T acc = T(0);
+        const int lo = Bf.off + ylo * sx;
+        const T* s_d = STAGED ? s_r + cap : cf + lo;
+        const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * Nf + lo;
+        const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * Nf + lo;
+        mg_stage_rhs<T, UPD, MG2_TPB>(MgRhs<T, UPD>{r, q, al}, rn, x, p, first, Bc, lo, ylo, sx, nst, c0, c1 - 1,
+                                      [&](int e, T bi) { s_b[e] = bi; });
+        if (!pend) {  // a system that converged at this iteration takes only the update of its cells
+            __syncthreads();
+            // x1 = x0 + w (b - A x0) / diag with x0 = (w / diag) b formed from the stage.  Cells of the outermost rows whose
+            // outer neighbour row is outside the stage get a value that no child reads.
+            int xx = x0;
+            for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
+                auto at = [](const T* a) { return STAGED ? *a : mg_coef(a); };
+                const int m = xx > 0 ? e - 1 : e + sx - 1, pp = xx + 1 < sx ? e + 1 : e - sx + 1;
+                const T rc = s_r[e], xi = rc * s_b[e];
+                T acc = at(s_d + e) * xi;
+                acc += at(s_cx + m) * (s_r[m] * s_b[m]);
+                acc += at(s_cx + e) * (s_r[pp] * s_b[pp]);
+                if (e >= sx) acc += at(s_cy + e - sx) * (s_r[e - sx] * s_b[e - sx]);
+                if (e + sx < nst) acc += at(s_cy + e) * (s_r[e + sx] * s_b[e + sx]);
+                s_x[e] = xi + rc * (s_b[e] - acc);
+                xx += dr;
+                if (xx >= sx) xx -= sx;
+            }
+            __syncthreads();
+            for (int l = c0 + (int)threadIdx.x; l < c1; l += MG2_TPB) {
+                const int Y = l / Bc.sx, X = l - Y * Bc.sx;
+                T acc = T(0);
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-            const int dx = ch & 1, dy = ch >> 1;
-            const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy;
-            if ((dx && !Bc.shx) || (dy && !Bc.shy) || xs >= sx || ys >= Bf.sy) continue;
-            const int c = (ys - ylo) * sx + xs;
-            acc += s_b[c] - mg2_apply<T, STAGED>(s_x, s_d, s_cx, s_cy, c, xs, sx, nst);
+                for (int ch = 0; ch < 4; ++ch) {
+                    const int dx = ch & 1, dy = ch >> 1;
+                    const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy;
+                    if ((dx && !Bc.shx) || (dy && !Bc.shy) || xs >= sx || ys >= Bf.sy) continue;
+                    const int c = (ys - ylo) * sx + xs;
+                    acc += s_b[c] - mg2_apply<T, STAGED>(s_x, s_d, s_cx, s_cy, c, xs, sx, nst);
+                }
+                bc[Bc.off + l] = acc;
+            }
         }
-        bc[tl.s0 + k] = acc;
+        if (c1 == cend) return;
+        c0 = c1;
+        fit();
+        __syncthreads();  // the stage is free
+        stage();
     }
 }
 
 // post-smoothing with the coarse correction, two sweeps: x1 (the pre-smoothed iterate of the restriction, recomputed)
 // on the tile and two halo rows, x' = x1 + s P e_c, the first sweep on the tile and one halo row, the second on the
 // tile.  DOT (finest level): partials of out.b, b.b, sum(out), sum(b) in the tile's MG_NW slots.  Stage: the tile and
-// three halo rows on each side (four arrays of
-// `cap` cells, three more when STAGED).
+// three halo rows on each side (four arrays of `cap` cells, three more when STAGED), or runs of the tile that fit.
 template <typename T, bool DOT, bool STAGED>
 __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_prolong2(
     pict_mg_level_t F, pict_mg_level_t C, const int32_t* tiles, const T* bv, const T* ec, T* out, T s, T w, double* part,
-    int cap, const double* sc) {
+    int cap, const double* sc, int* err) {
     constexpr int MG2_TPB = Mg2<STAGED>::threads;
     extern __shared__ __align__(16) unsigned char mg_stage_raw[];
     __shared__ double s_red[MG2_TPB / 32][4];
@@ -764,65 +791,93 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_pro
     w = mg_weight(Bf, w);
     const T* __restrict__ cf = reinterpret_cast<const T*>(F.coef);
     const int N = F.num_cells, sx = Bf.sx, nf = sx * Bf.sy;
-    const int lo = max(Bf.off, tl.s0 - 3 * sx), hi = min(Bf.off + nf, tl.s0 + tl.cnt + 3 * sx), nst = hi - lo;
-    if (nst > cap) return;  // as k_mg_restrict2
+    // the cells [s0, s1) of the tile at a time, with the stage cells [lo, lo + nst)
+    const int send = tl.s0 + tl.cnt;
+    int s0 = tl.s0, s1, lo, nst;
+    auto range = [&] {
+        lo = max(Bf.off, s0 - 3 * sx);
+        nst = min(Bf.off + nf, s1 + 3 * sx) - lo;
+    };
+    auto fit = [&] {
+        s1 = send;
+        range();
+        if (nst > cap) {
+            s1 = min(send, s0 + max(cap - 6 * sx, 1));
+            range();
+        }
+    };
+    fit();
     T* s_x = reinterpret_cast<T*>(mg_stage_raw);  // x0, then the first post sweep
     T* s_y = s_x + cap;                           // s P e_c, then x'
     T* s_b = s_y + cap;
     T* s_r = s_b + cap;
-    mg2_stage_stencil<T, STAGED>(cf, N, lo, nst, w, s_r, s_r + cap, s_r + 2 * cap, s_r + 3 * cap);
-    const T* s_d = STAGED ? s_r + cap : cf + lo;
-    const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * N + lo;
-    const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * N + lo;
+    auto stage = [&] {
+        if (nst <= cap) mg2_stage_stencil<T, STAGED>(cf, N, lo, nst, w, s_r, s_r + cap, s_r + 2 * cap, s_r + 3 * cap);
+    };
+    stage();
     const int dq = MG2_TPB / sx, dr = MG2_TPB - dq * sx;
     mg_pdl_wait();
     mg_pdl_next();
     if (mg_done(sc, tl.sys)) return;
-    {
-        const int l = lo - Bf.off + (int)threadIdx.x;
-        int y = l / sx, x = l - y * sx;
-        for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
-            const T b = bv[lo + e];
-            s_y[e] = s * ec[Bc.off + (x >> Bc.shx) + Bc.sx * (y >> Bc.shy)];
-            s_b[e] = b;
-            s_x[e] = s_r[e] * b;  // written by this thread
-            x += dr;
-            y += dq;
-            if (x >= sx) {
-                x -= sx;
-                ++y;
+    double a = 0.0, c2 = 0.0, sz = 0.0, sr = 0.0;
+    for (;;) {
+        if (nst > cap) {  // a block wider than the level announced
+            if (threadIdx.x == 0) *err = 1;
+            break;
+        }
+        const T* s_d = STAGED ? s_r + cap : cf + lo;
+        const T* s_cx = STAGED ? s_r + 2 * cap : cf + (size_t)2 * N + lo;
+        const T* s_cy = STAGED ? s_r + 3 * cap : cf + (size_t)4 * N + lo;
+        {
+            const int l = lo - Bf.off + (int)threadIdx.x;
+            int y = l / sx, x = l - y * sx;
+            for (int e = threadIdx.x; e < nst; e += MG2_TPB) {
+                const T b = bv[lo + e];
+                s_y[e] = s * ec[Bc.off + (x >> Bc.shx) + Bc.sx * (y >> Bc.shy)];
+                s_b[e] = b;
+                s_x[e] = s_r[e] * b;  // written by this thread
+                x += dr;
+                y += dq;
+                if (x >= sx) {
+                    x -= sx;
+                    ++y;
+                }
             }
         }
+        __syncthreads();
+        // stage cells [k0, k1): f(stage cell, its column)
+        auto cells = [&](int k0, int k1, auto&& f) {
+            int x = (lo - Bf.off + k0 + (int)threadIdx.x) % sx;
+            for (int c = k0 + (int)threadIdx.x; c < k1; c += MG2_TPB) {
+                f(c, x);
+                x += dr;
+                if (x >= sx) x -= sx;
+            }
+        };
+        const int t0 = s0 - lo, t1 = s1 - lo;
+        cells(max(0, t0 - 2 * sx), min(nst, t1 + 2 * sx),
+              [&](int c, int x) { s_y[c] += mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+        __syncthreads();
+        cells(max(0, t0 - sx), min(nst, t1 + sx),
+              [&](int c, int x) { s_x[c] = mg2_sweep<T, STAGED>(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+        __syncthreads();
+        cells(t0, t1, [&](int c, int x) {
+            const T zi = mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst);
+            out[lo + c] = zi;
+            if (DOT) {
+                const double bi = (double)s_b[c];
+                a += bi * (double)zi;
+                c2 += bi * bi;
+                sz += (double)zi;
+                sr += bi;
+            }
+        });
+        if (s1 == send) break;
+        s0 = s1;
+        fit();
+        __syncthreads();  // the stage is free
+        stage();
     }
-    __syncthreads();
-    // stage cells [c0, c1): f(stage cell, its column)
-    auto cells = [&](int c0, int c1, auto&& f) {
-        int x = (lo - Bf.off + c0 + (int)threadIdx.x) % sx;
-        for (int c = c0 + (int)threadIdx.x; c < c1; c += MG2_TPB) {
-            f(c, x);
-            x += dr;
-            if (x >= sx) x -= sx;
-        }
-    };
-    const int t0 = tl.s0 - lo, t1 = t0 + tl.cnt;
-    cells(max(0, t0 - 2 * sx), min(nst, t1 + 2 * sx),
-          [&](int c, int x) { s_y[c] += mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
-    __syncthreads();
-    cells(max(0, t0 - sx), min(nst, t1 + sx),
-          [&](int c, int x) { s_x[c] = mg2_sweep<T, STAGED>(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
-    __syncthreads();
-    double a = 0.0, c2 = 0.0, sz = 0.0, sr = 0.0;
-    cells(t0, t1, [&](int c, int x) {
-        const T zi = mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst);
-        out[lo + c] = zi;
-        if (DOT) {
-            const double bi = (double)s_b[c];
-            a += bi * (double)zi;
-            c2 += bi * bi;
-            sz += (double)zi;
-            sr += bi;
-        }
-    });
     if (DOT) {
         a = mg_warp_sum(a);
         c2 = mg_warp_sum(c2);
@@ -1603,17 +1658,20 @@ static pict_status_t run_pcg_mg(const pict_domain_t* dom, const pict_mg_level_t*
     if (nu[0] == 2 && dom->tile_cells + 6 * levels[0].max_block_sx > (3 * cap) / 4) nu[0] = 1;
     const int nu_sub = g_mg_sweeps >= 2 ? 2 : 1;
     // shared-memory stages of the 2D restriction / prolongation.  One sweep: x0 (or x'), b, diag of MG_STAGE cells.  Two
-    // sweeps: what the level's tiles need at most, so that small blocks leave room for more CTAs on an SM: a coarse
-    // tile of at most MG_TILE cells has at most (4 MG_TILE + 8 sx) fine cells with two halo rows on each side (rows
-    // that it covers partly included), a tile of the level its own cells and six rows.
+    // sweeps: what tiles of MG_TILE cells need at most, so that small blocks leave room for more CTAs on an SM: a coarse
+    // tile of MG_TILE cells has at most (4 MG_TILE + 8 sx) fine cells with two halo rows on each side (rows that it covers
+    // partly included), a tile of the level its own cells and six rows.  Other tile sizes give the same results: a larger
+    // tile is walked in runs that fit.  (The whole stage that two sweeps promise, 4096 cells, everywhere: cavities_16 4.91
+    // -> 5.25 ms, cavities_256 22.98 -> 23.6.)
     const size_t stage3 = D == 2 ? 3 * (size_t)MG_STAGE * sizeof(T) : 0;
     int cap_r[16], cap_p[16];
     size_t sm_r[16], sm_p[16];
     bool staged_r[16], staged_p[16];
     for (int l = 0; l < nl; ++l) {
-        const int sx = levels[l].max_block_sx, tile = l == 0 ? dom->tile_cells : MG_TILE;
+        const int sx = levels[l].max_block_sx;
+        if (sx <= 0 || 6 * sx >= (3 * MG_STAGE) / 4) nu[l] = 1;  // rows too long for two sweeps with any tile, or unknown
         cap_r[l] = 4 * MG_TILE + 8 * sx < MG_STAGE ? 4 * MG_TILE + 8 * sx : MG_STAGE;
-        cap_p[l] = tile + 6 * sx;
+        cap_p[l] = (l == 0 ? dom->tile_cells : MG_TILE) + 6 * sx;
         // the couplings too where a launch is about one wave of CTAs, whose latency counts; with several waves the
         // kernels are bound by throughput and more CTAs on an SM hide more (256 cavities: finest prolongation 69 us
         // staged, 48..55 not; 16 cavities: 8.3 us staged)
@@ -1664,7 +1722,7 @@ static pict_status_t run_pcg_mg(const pict_domain_t* dom, const pict_mg_level_t*
                 mg_launch(staged_r[l] ? (u ? k_mg_restrict2<T, true, true> : k_mg_restrict2<T, false, true>)
                                       : (u ? k_mg_restrict2<T, true, false> : k_mg_restrict2<T, false, false>),
                           C.num_tiles, staged_r[l] ? Mg2<true>::threads : Mg2<false>::threads, sm_r[l], st, F, C, src, u ? q : nullptr, u ? rn : nullptr, u ? xout : nullptr, u ? p : nullptr, sc, first, lb[l + 1], wj,
-                          cap_r[l]);
+                          cap_r[l], err);
             else
                 mg_launch(u ? k_mg_restrict<T, D, true> : k_mg_restrict<T, D, false>, C.num_tiles, MG_TPB, stage3, st, F, C, src,
                           u ? q : nullptr, u ? rn : nullptr, u ? xout : nullptr, u ? p : nullptr, u ? sc : nullptr, first,
@@ -1682,7 +1740,7 @@ static pict_status_t run_pcg_mg(const pict_domain_t* dom, const pict_mg_level_t*
                                       : (dot ? k_mg_prolong2<T, true, false> : k_mg_prolong2<T, false, false>),
                           tiles, staged_p[l] ? Mg2<true>::threads : Mg2<false>::threads, sm_p[l], st, levels[l], levels[l + 1],
                           tab, dot ? rnew : lb[l], lx[l + 1], dot ? z : lx[l], sp, wj, dot ? part : nullptr,
-                          cap_p[l], sc);
+                          cap_p[l], sc, err);
             else
                 mg_launch(dot ? k_mg_prolong<T, D, true> : k_mg_prolong<T, D, false>, tiles, MG_TPB, stage3, st, levels[l],
                           levels[l + 1], tab, dot ? rnew : lb[l], lx[l + 1], dot ? z : lx[l], sp, wj, dot ? part : nullptr,

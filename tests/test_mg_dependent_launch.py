@@ -2,7 +2,8 @@
 not provoked on a GPU).  Every operand that a kernel of the loop writes must be read after griddepcontrol.wait: a
 parameter that is declared __restrict__ and only read counts as constant during the kernel, so its load may take the
 read-only path and be moved across the wait.  Stencils and tables, which no kernel of the loop writes, are read with
-__ldg or through local pointers."""
+__ldg or through local pointers.  And no CTA leaves before the wait: a kernel's reads before its own wait rest on every
+CTA of its predecessor having waited."""
 import os
 import re
 
@@ -56,6 +57,14 @@ def test_loop_kernels_are_found():
 def test_no_operand_is_declared_read_only(name):
     params, _ = _loop_kernels()[name]
     assert "__restrict__" not in params
+
+
+@pytest.mark.parametrize("name", sorted(_loop_kernels()))
+def test_no_return_before_the_wait(name):
+    _, body = _loop_kernels()[name]
+    wait = re.search(r"\bmg_pdl_(?:entry|wait)\(\);", body)
+    assert wait, "does not wait for its predecessor"
+    assert not re.search(r"\breturn\b", body[:wait.start()])
 
 
 def test_no_member_of_an_operand_struct_is_declared_read_only():
