@@ -620,12 +620,13 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
 }
 
 // ---------------------------------------------------------------------------------------------
-// The two-sweep tile kernels (2D, no y-periodic block).  A CTA of MG2_TPB threads holds the rows of its tile and the
+// The two-sweep tile kernels (2D, no y-periodic block).  A CTA holds the rows of its tile and the
 // halo rows of the sweeps in shared memory: w / diag and the +x and +y couplings (the operator is symmetric, so a
 // cell's -x and -y couplings are its neighbours' and five coefficients become three), the right-hand side and two
 // iterates.  The stencil is staged before the wait on the predecessor (mg_pdl_wait), so what is left of a kernel's own
-// chain is one read of the right-hand side and the sweeps in shared memory.  A coupling across a fixed face is 0, which
-// masks its term: -x of the first cell of a row reads the +x coupling of the row's last cell, the periodic one or 0.
+// chain is one read of the right-hand side and the sweeps in shared memory.  The -x coupling of a row's first
+// cell is the +x coupling of its last one, taken on periodic rows only: what a stencil holds at a face without a neighbour
+// has no meaning.
 //
 // What bounds them: on few systems the latency of this chain (a level is a few CTAs), on many the shared-memory
 // reads of the sweeps over tile and halo.  Per launch of the finest level, before (256 threads, everything but b and the
@@ -641,12 +642,12 @@ constexpr int MG_TILE = 512;  // cells of a tile that the stages hold whole (the
 // (A v) at stage cell c (column x of rows of sx, stage of nst cells).  The diagonal term is kept beside the others and
 // not folded into a (1 - w) v, so that what is left of a constant v cancels here and is not carried through the sweeps.
 template <typename T, bool STAGED>
-__device__ __forceinline__ T mg2_apply(const T* v, const T* d, const T* cx, const T* cy, int c, int x, int sx, int nst) {
+__device__ __forceinline__ T mg2_apply(const T* v, const T* d, const T* cx, const T* cy, int c, int x, int sx, int px, int nst) {
     auto at = [](const T* a) { return STAGED ? *a : mg_coef(a); };
     const int m = x > 0 ? c - 1 : c + sx - 1, p = x + 1 < sx ? c + 1 : c - sx + 1;
     T acc = at(d + c) * v[c];
-    acc += at(cx + m) * v[m];
-    acc += at(cx + c) * v[p];
+    acc += x > 0 || px ? at(cx + m) * v[m] : T(0);
+    acc += x + 1 < sx || px ? at(cx + c) * v[p] : T(0);
     if (c >= sx) acc += at(cy + c - sx) * v[c - sx];
     if (c + sx < nst) acc += at(cy + c) * v[c + sx];
     return acc;
@@ -655,8 +656,8 @@ __device__ __forceinline__ T mg2_apply(const T* v, const T* d, const T* cx, cons
 // one damped-Jacobi sweep there: v + r (b - A v) with r = w / diag
 template <typename T, bool STAGED>
 __device__ __forceinline__ T mg2_sweep(const T* v, const T* b, const T* r, const T* d, const T* cx, const T* cy, int c, int x,
-                                       int sx, int nst) {
-    return v[c] + r[c] * (b[c] - mg2_apply<T, STAGED>(v, d, cx, cy, c, x, sx, nst));
+                                       int sx, int px, int nst) {
+    return v[c] + r[c] * (b[c] - mg2_apply<T, STAGED>(v, d, cx, cy, c, x, sx, px, nst));
 }
 
 template <bool STAGED>
@@ -744,8 +745,8 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
                 const int m = xx > 0 ? e - 1 : e + sx - 1, pp = xx + 1 < sx ? e + 1 : e - sx + 1;
                 const T rc = s_r[e], xi = rc * s_b[e];
                 T acc = at(s_d + e) * xi;
-                acc += at(s_cx + m) * (s_r[m] * s_b[m]);
-                acc += at(s_cx + e) * (s_r[pp] * s_b[pp]);
+                acc += xx > 0 || Bf.px ? at(s_cx + m) * (s_r[m] * s_b[m]) : T(0);
+                acc += xx + 1 < sx || Bf.px ? at(s_cx + e) * (s_r[pp] * s_b[pp]) : T(0);
                 if (e >= sx) acc += at(s_cy + e - sx) * (s_r[e - sx] * s_b[e - sx]);
                 if (e + sx < nst) acc += at(s_cy + e) * (s_r[e + sx] * s_b[e + sx]);
                 s_x[e] = xi + rc * (s_b[e] - acc);
@@ -762,7 +763,7 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_res
                     const int xs = (X << Bc.shx) + dx, ys = (Y << Bc.shy) + dy;
                     if ((dx && !Bc.shx) || (dy && !Bc.shy) || xs >= sx || ys >= Bf.sy) continue;
                     const int c = (ys - ylo) * sx + xs;
-                    acc += s_b[c] - mg2_apply<T, STAGED>(s_x, s_d, s_cx, s_cy, c, xs, sx, nst);
+                    acc += s_b[c] - mg2_apply<T, STAGED>(s_x, s_d, s_cx, s_cy, c, xs, sx, Bf.px, nst);
                 }
                 bc[Bc.off + l] = acc;
             }
@@ -856,13 +857,13 @@ __global__ void __launch_bounds__(Mg2<STAGED>::threads, STAGED ? 2 : 4) k_mg_pro
         };
         const int t0 = s0 - lo, t1 = s1 - lo;
         cells(max(0, t0 - 2 * sx), min(nst, t1 + 2 * sx),
-              [&](int c, int x) { s_y[c] += mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+              [&](int c, int x) { s_y[c] += mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, Bf.px, nst); });
         __syncthreads();
         cells(max(0, t0 - sx), min(nst, t1 + sx),
-              [&](int c, int x) { s_x[c] = mg2_sweep<T, STAGED>(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst); });
+              [&](int c, int x) { s_x[c] = mg2_sweep<T, STAGED>(s_y, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, Bf.px, nst); });
         __syncthreads();
         cells(t0, t1, [&](int c, int x) {
-            const T zi = mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, nst);
+            const T zi = mg2_sweep<T, STAGED>(s_x, s_b, s_r, s_d, s_cx, s_cy, c, x, sx, Bf.px, nst);
             out[lo + c] = zi;
             if (DOT) {
                 const double bi = (double)s_b[c];

@@ -156,3 +156,29 @@ def test_rows_too_long_for_two_sweeps(announced, dtype):
     # the recursion's residual plus the rounding of its at most 100 updates at the largest row sum and iterate
     drift = 100 * torch.finfo(dtype).eps * abs(A).sum(axis=1).max() * float(x.abs().max())
     assert np.sqrt((r ** 2).mean()) <= tol + drift
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("copies", [0, 140])
+def test_couplings_across_fixed_faces_are_not_read(copies, dtype):
+    """A face without a neighbour has no term, whatever its coefficient holds: NaN there changes no bit of the solution."""
+    from pict_b200.batch import BatchDomain
+    from pict_b200.engine import PISOStepper
+    from pict_b200.multigrid import hierarchy_for
+    specs = [lid_cavity(100, viscosity=1e-3), lid_cavity(37, viscosity=1e-3), _channel(64, 48)]
+    specs += [specs[0]] * copies
+    b = BatchDomain([build_product(s, dtype) for s in specs], time_steps=[0.005] * len(specs))
+    PISOStepper(b, time_step=0.005, advection_tol=1e-8, pressure_tol=1e-8).step()
+    mg = hierarchy_for(b)
+    assert mg.levels[0].sweeps == 2
+    g = torch.Generator(device="cpu").manual_seed(13)
+    rhs = torch.randn(b.getTotalSize(), generator=g, dtype=dtype).cuda()
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    out = []
+    for poison in (False, True):
+        coef = b.P.coef.clone().reshape(5, -1)
+        if poison:
+            coef[1:][b._nbr.reshape(4, -1) < 0] = float("nan")
+        mg.setup(coef, st)
+        out.append(_mg_solve(b, mg, rhs, iterations=3)[0])
+    assert bool(torch.isfinite(out[0]).all()) and torch.equal(out[0], out[1])
