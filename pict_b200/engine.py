@@ -413,20 +413,40 @@ class PISOStepper:
         return [[P.decode_infos(t) for t in row] for row in self.info_r]
 
     def check(self):
-        """Raise LinsolveError if any solve of the last step failed (synchronises)."""
+        """Raise LinsolveError if any solve of the last step failed (synchronises).  The message names the first
+        failed solve like the reference's wrapper, then every failed one with its system (the batch's member and
+        its block sizes), tolerance, residual, iterations and status."""
         adv, ps = self.infos()
-        extra = [("pressure %d refinement %d" % (k, m), r) for k, row in enumerate(self.refine_infos())
+        extra = [("pressure %d refinement %d" % (k, m), r, 1, self.refine_tol) for k, row in enumerate(self.refine_infos())
                  for m, r in enumerate(row)]
-        first = [("pressure %d" % k, p) for k, p in enumerate(ps)] if self.pressure_first_solve else []
-        for name, lst in [("advection", adv)] + first + extra:
+        first = [("pressure %d" % k, p, 1, self.p_tol) for k, p in enumerate(ps)] if self.pressure_first_solve else []
+        head, failed = None, []
+        for name, lst, nrhs, tol in [("advection", adv, self.dims, self.adv_tol)] + first + extra:
             for i, inf in enumerate(lst):
                 if getattr(inf, "status", 0) == 1:
-                    raise LinsolveError("%s solve: inter-CTA barrier timed out (system %d)" % (name, i))
-                if not inf.isFiniteResidual:
-                    raise LinsolveError("%s solve reported non-finite residual for RHS %d: %s" % (name, i, inf))
-                if not inf.converged:
-                    raise LinsolveError("%s solve RHS %d did not converge: %s" % (name, i, inf))
+                    what = "%s solve: a wait of the kernel gave up (system %d)" % (name, i // nrhs)
+                elif not inf.isFiniteResidual:
+                    what = "%s solve reported non-finite residual for RHS %d: %s" % (name, i, inf)
+                elif not inf.converged:
+                    what = "%s solve RHS %d did not converge: %s" % (name, i, inf)
+                else:
+                    continue
+                head = head or what
+                failed.append("%s, %s, tolerance %g, residual %g after %d iterations, status %d" % (
+                    name, self._system_name(i // nrhs), tol, inf.finalResidual, inf.usedIterations,
+                    getattr(inf, "status", 0)))
+        if failed:
+            shown = failed[:8] + (["and %d more" % (len(failed) - 8)] if len(failed) > 8 else [])
+            raise LinsolveError("%s\n%d failed of the last step:\n  %s" % (head, len(failed), "\n  ".join(shown)))
         return adv, ps
+
+    def _system_name(self, s):
+        """System s of the solver reports for a message: the batch's member it is, and its block sizes."""
+        d = self.domain
+        member = d.order[s] if hasattr(d, "order") else None
+        dom = d if member is None else d.domains[member]
+        sizes = ", ".join("x".join(str(n) for n in reversed(b.velocity.shape[2:])) for b in dom.getBlocks())
+        return "system %d (%s%s)" % (s, "" if member is None else "member %d, " % member, sizes)
 
     # ---------------- CUDA graph ----------------
     def capture(self, steps: int = 1, time_step=None):
