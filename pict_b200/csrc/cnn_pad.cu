@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(PAD_THREADS) k_mb_pad_gather(int n, int bc, co
 
 // gsrc[sb][bc][loc] = sum over the readers k of source cell g = (sb, loc) of gout[ob_k][bc][pos_k].  Away from the
 // connections a cell has one reader, the padded cell over itself, whose place is kept in registers; the others
-// follow in the list's order.
+// follow in the list's order.  The sum starts from +0, as an index_add into zeros does (a -0 comes out as +0).
 template <typename T>
 __global__ void __launch_bounds__(PAD_THREADS) k_mb_pad_scatter_sum(int n, int bc, const int32_t* __restrict__ sb,
                                                                     const int32_t* __restrict__ loc,
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(PAD_THREADS) k_mb_pad_scatter_sum(int n, int b
     for (; c + (PAD_U - 1) * step < bc; c += PAD_U * step) {
         T v[PAD_U];
 #pragma unroll
-        for (int u = 0; u < PAD_U; ++u) v[u] = from[(size_t)(c + u * step) * os];
+        for (int u = 0; u < PAD_U; ++u) v[u] = T(0) + from[(size_t)(c + u * step) * os];
         for (int k = k0 + 1; k < k1; ++k) {
             const T* __restrict__ more = gout.p[rob[k]] + rpos[k];
             const int64_t ms = gout.n[rob[k]];
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(PAD_THREADS) k_mb_pad_scatter_sum(int n, int b
         for (int u = 0; u < PAD_U; ++u) dst[(size_t)(c + u * step) * ss] = v[u];
     }
     for (; c < bc; c += step) {
-        T v = from[(size_t)c * os];
+        T v = T(0) + from[(size_t)c * os];
         for (int k = k0 + 1; k < k1; ++k) v += gout.p[rob[k]][(size_t)c * gout.n[rob[k]] + rpos[k]];
         dst[(size_t)c * ss] = v;
     }

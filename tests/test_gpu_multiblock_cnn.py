@@ -59,3 +59,40 @@ def test_padding_kernels_equal_the_index_map(name, k):
     for a, b in zip(*grads):
         assert torch.allclose(a, b, rtol=1e-13, atol=1e-13)
     assert _lib.load() is not None
+
+
+@pytest.mark.parametrize("channels", [64, 67])
+def test_padding_kernels_with_many_channels_a_thread(channels):
+    """Blocks so large that a thread walks 32 channels of its cell and more, eight at a time with a remainder (small
+    blocks give every channel its own thread): the padded values bitwise, the gradient to round-off, at the connections
+    of a 2 x 2 grid of uneven blocks too; a gradient of -0 gives +0, as adding it to zeros does."""
+    from pict_b200 import PISOtorch as P
+    dom = P.Domain(2, torch.tensor([1e-3]), name="grid", dtype=torch.float32, device=torch.device("cuda"),
+                   passiveScalarChannels=0)
+    sizes = [(320, 330), (320, 325), (323, 330), (323, 325)]   # (y, x) per block
+    b = [dom.CreateBlockWithSize(P.Int4(x, y, 1, 2), name="b%d" % i) for i, (y, x) in enumerate(sizes)]
+    for blk in b:
+        blk.CloseAllBoundaries()
+    b[0].ConnectBlock("+x", b[1], "-x", "-y")
+    b[0].ConnectBlock("+y", b[2], "-y", "-x")
+    b[1].ConnectBlock("+y", b[3], "-y", "-x")
+    b[2].ConnectBlock("+x", b[3], "-x", "-y")
+    layer = MultiblockConv(dom, "ZERO", channels, 1, 3, dtype=torch.float32)
+    g = torch.Generator().manual_seed(5)
+    xs = [torch.randn((1, channels) + s, generator=g) for s in sizes]
+    ws = [torch.randn((1, channels, s[0] + 2, s[1] + 2), generator=g) for s in sizes]
+    res = []
+    for dev in ("cpu", "cuda"):
+        layer = layer.to(dev)
+        x = [t.detach().clone().to(dev).requires_grad_(True) for t in xs]
+        pads = layer.pad(x)
+        torch.autograd.backward(pads, [w.to(dev) for w in ws])
+        res.append(([p.detach().cpu() for p in pads], [t.grad.cpu() for t in x]))
+    for a, c in zip(res[0][0], res[1][0]):
+        assert torch.equal(a, c)
+    for a, c in zip(res[0][1], res[1][1]):
+        # at most 4 readers a cell, summed in another order: 3 roundings of a sum of 4 values
+        assert float((a - c).abs().max()) <= 3 * 4 * 2 ** -24 * float(max(w.abs().max() for w in ws))
+    x = [t.detach().clone().cuda().requires_grad_(True) for t in xs]
+    torch.autograd.backward(layer.pad(x), [torch.full_like(w, -0.0).cuda() for w in ws])
+    assert not any(bool(torch.signbit(t.grad).any()) for t in x)
