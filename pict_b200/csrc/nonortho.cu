@@ -231,8 +231,8 @@ __device__ __forceinline__ T lap(const T* tr, int c1, int c2) {
 
 // ---------------------------------------------------------------------------------------------
 // Cells away from walls and connections.  Along every axis such a cell has both neighbours inside its block (the
-// wrapped one on a periodic axis of at least two cells), so every corner is the mean of its four cells: the walk
-// around it need not be made, the own and the face neighbour's shares of the two corners of a tangential axis cancel,
+// wrapped one on a periodic axis of at least three cells, the shortest that a domain takes), so every corner is the mean
+// of its four cells: the walk around it need not be made, the own and the face neighbour's shares of the two corners of a tangential axis cancel,
 // and with them the own cell's coefficient.  What remains per pair of axes is read directly: the off-diagonal
 // coefficients of the 2 D neighbours, and for the right-hand sides the four diagonal cells.  The kernels
 // k_nonortho_plain_* take these cells and the walking kernels the others.  Measured on 96 x 65 x 80 periodic cells in
@@ -251,7 +251,7 @@ __device__ __forceinline__ bool plain_cell(const pict_block_t& B, const int* p, 
         const bool lo = p[a] > 0, hi = p[a] < s - 1;
         off[2 * a] = lo ? -stride[a] : (s - 1) * stride[a];
         off[2 * a + 1] = hi ? stride[a] : -(s - 1) * stride[a];
-        if (!(lo && hi) && !(s >= 2 && B.face[2 * a].type == PICT_FACE_PERIODIC && B.face[2 * a + 1].type == PICT_FACE_PERIODIC))
+        if (!(lo && hi) && !(s >= 3 && B.face[2 * a].type == PICT_FACE_PERIODIC && B.face[2 * a + 1].type == PICT_FACE_PERIODIC))
             plain = false;
     }
     return plain;
