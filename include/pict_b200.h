@@ -147,7 +147,8 @@ typedef struct pict_solve_params {
     int32_t transpose;         /* solve with A^T (adjoint solves) */
     int32_t convergence;       /* PICT_CONV_* (ComputeConvergenceCriterion, extensions/cg_solver_kernel.cu:77-110);
                                   the ABS criteria with CG only (classic order) */
-    int32_t group_size;        /* upper bound of CTAs of the persistent launch (0: automatic) */
+    int32_t group_size;        /* upper bound of CTAs of the persistent launch (0: automatic); solves that take
+                                  thread-block clusters (pict_krylov_set_cluster_mode) do not use it */
     int32_t threads;           /* threads per CTA (0: automatic) */
     int32_t subtract_mean;     /* 1: x -= mean(x) per system after the solve (PISOtorch_simulation.py:1243-1244) */
     int32_t write_block_pressure; /* 1: also copy x into the blocks' pressure (CopyPressureResultToBlocks) */
@@ -249,15 +250,21 @@ pict_status_t pict_solve(const pict_domain_t* dom, const void* coef, const void*
                          const pict_solve_params_t* params, void* info_out, void* workspace,
                          int64_t workspace_bytes, void* stream);
 
-/* Process-wide choice of the launch form of the single-reduction CG (variant 1; no counterpart in the
- * reference) and of BiCGStab: 1 (default) solves each system with one thread-block cluster (16 CTAs, else 8) when a
- * domain holds few systems (at most 8) of at most 262,144 cells, reducing the inner products through
- * distributed shared memory with no grid-wide barrier (systems of up to 65,536 cells FP32 or 32,768 FP64, BiCGStab 16,384
- * to 32,768 by type and components, with every vector in registers; BiCGStab above that takes the grid); 0 always
- * uses the persistent grid; 2 uses clusters whenever they fit. */
+/* Process-wide choice of the launch form of the single-reduction CG (variant 1, NORM2 criteria, no restarts; no
+ * counterpart in the reference) and of BiCGStab (variant 0, NORM2 criteria):
+ * 1 (default): a domain of at most 8 systems is solved by one thread-block cluster per system, reducing the inner
+ *   products through distributed shared memory with no grid-wide barrier.  The largest system decides: CG of up to
+ *   65,536 cells FP32 or 32,768 FP64, BiCGStab of one or two components of up to 32,768 FP32 or 16,384 FP64 and of three
+ *   of up to 16,384 keep every vector in registers (16 CTAs a cluster); larger CG of up to 262,144 cells takes clusters
+ *   of 16 CTAs, else 8, with the vectors in memory; everything else takes the persistent grid.
+ * 0: always the persistent grid.  2: clusters whenever they fit, for any number of systems.
+ * Cluster solves do not use pict_solve_params_t.group_size.  The forms sum in different orders: on the grid, and among
+ * on-chip solves, a system's result does not depend bit for bit on the other systems of its batch or on the launch, but
+ * with the default choice it changes within the tolerance (and its iteration count by one or two) where a ninth system or
+ * one above the limits joins the batch.  Mode 0 gives results that do not depend on the batch. */
 void pict_krylov_set_cluster_mode(int32_t mode);
-/* BiCGStab kernel (no counterpart in the reference): 0 (default) four grid barriers per iteration for every
- * solve; 1 two barriers per iteration (NORM2 / NORM2_NORMALIZED criteria, up to two right-hand sides per launch;
+/* BiCGStab kernel (no counterpart in the reference): 0 (default) the cluster form where pict_krylov_set_cluster_mode
+ * selects it, else four grid barriers per iteration; 1 (on the grid always) two barriers per iteration (NORM2 / NORM2_NORMALIZED criteria, up to two right-hand sides per launch;
  * the half step forms s on the fly, the full step forms the next search direction on the fly with rho' from the
  * recurrence rw.r - alpha rw.v - omega rw.t) with one CTA per SM, 2 the same with two CTAs per SM.  All follow
  * bicgstabSolveGPU's iteration and reports.  Variants 1 and 2 take one more workspace vector per right-hand side
@@ -343,8 +350,9 @@ void pict_mg_set_smoothing_sweeps(int32_t sweeps);
  * the iterations the systems need; 0 captures the fixed sequence of `iterations` iterations. */
 void pict_mg_set_graph_loop(int32_t enable);
 /* Process-wide choice (no counterpart in the reference): 1 (default) the kernels of pict_pcg_mg are launched with
- * programmatic stream serialization (each one waits for its predecessor's writes at its first instruction and lets
- * the next one launch at once, so launch latency overlaps the predecessor's last CTAs); 0 plain launches. */
+ * programmatic stream serialization (each one waits for its predecessor's writes before it touches anything a kernel of
+ * the loop writes, reading its tables and stencils ahead of the wait, and then lets the next one launch, so launch latency
+ * and those reads overlap the predecessor); 0 plain launches.  Same results bit for bit. */
 void pict_mg_set_dependent_launch(int32_t enable);
 /* Galerkin coarse operator R A P of `fine` into coarse->coef (aggregates of 2^D cells). */
 pict_status_t pict_mg_galerkin(const pict_mg_level_t* fine, const pict_mg_level_t* coarse, void* stream);

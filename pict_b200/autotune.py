@@ -1,8 +1,8 @@
 """Autotuner of the persistent Krylov launch shapes.
 
 Tunables: the work-tile size of the Krylov kernels (cells per tile, 512..2048), the upper bound of
-co-resident CTAs of a persistent launch (0 = every CTA the occupancy allows, or one CTA per SM) and
-the CG recurrence (0: the reference's two-reduction order, 1: single reduction).  Each candidate is
+co-resident CTAs of a persistent launch (0 = every CTA the occupancy allows, or one CTA per SM; solves of
+few small systems, which take thread-block clusters, do not use either) and the CG recurrence (0: the reference's two-reduction order, 1: single reduction).  Each candidate is
 timed on the real PISO step of the domain (CUDA events, after warm-up steps, from the same saved
 state), and the fastest is applied.  Results are cached in a JSON file keyed by a signature of the
 workload (dimensions, dtype, block sizes, solver settings, device), so later runs reuse them.

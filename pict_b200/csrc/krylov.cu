@@ -17,7 +17,7 @@
 //    kernel records an error and returns;
 //  * inner products are accumulated in FP64, reduced per tile inside the CTA
 //    and then per system over the tile partials in a fixed order, so results do
-//    not depend on the number of CTAs and are bitwise reproducible;
+//    not depend on the number of CTAs or on the other systems of the launch and are bitwise reproducible;
 //  * the stencil SpMV reads structured neighbours directly (i +- stride) and
 //    uses the precomputed neighbour table only on block faces; the search
 //    direction is formed on the fly for the neighbours (double buffered), so
@@ -25,6 +25,10 @@
 //  * BiCGStab advances all right-hand sides of a system (the D velocity
 //    components) together, sharing the matrix loads, each with its own scalars
 //    and convergence state.
+//
+// Domains of few systems are solved by one thread-block cluster per system instead
+// (pict_krylov_set_cluster_mode): on chip where the largest fits (krylov_resident.cuh), else CG with
+// the vectors in memory (k_cg1_cluster).
 //
 // Iteration semantics, stopping rule and reported iteration counts follow the
 // reference: CG extensions/cg_solver_kernel.cu:236-427, BiCGStab extensions/bicgstab_solver_kernel.cu:240-360, convergence criterion
@@ -215,7 +219,10 @@ __device__ void load_slots(const pict_domain_t& dom, TileSlots& S) {
     __syncthreads();
 }
 
-// Tiles of a system above which its partials are summed by the whole CTA instead of one warp.
+// Tiles of a system above which its partials are summed by the whole CTA instead of one warp.  One system, us an
+// iteration, CTA / warp: 32 tiles 6.69 / 6.62 (CG) and 24.3 / 23.6 (BiCGStab, two components), 64 tiles 6.55 / 6.77 and
+// 24.3 / 24.8, 128 tiles 6.6 / 7.5 and 24.6 / 28.2, 256 tiles 8.3 / 10.3 and 29.8 / 38.5, 1728 tiles 30 / 48 and
+// 89 / 219.  They cross at 64 tiles; up to 256 the warp's order, and so the bits of smaller systems, was kept.
 constexpr int KR_WIDE = 256;
 
 // Sum the tile partials of each slot's system (fixed order) into out[slot][k].  Only slots whose bit is set in `mask`
@@ -1932,13 +1939,14 @@ static size_t workspace_total(const pict_domain_t* dom, const pict_solve_params_
 
 // 0: persistent grid only; 1: clusters where they apply (default); 2: clusters whenever possible
 static int g_cluster_mode = 1;
-// BiCGStab kernel: 0 (default) the four-barrier form for every solve; 1 the two-barrier form (NORM2
-// criteria, up to two right-hand sides per launch) with one 512-thread CTA per SM and 128 registers per
-// thread, 2 the same with two CTAs per SM (64 registers, some spilled).  Measured on the batch of 256
-// cavities (mixed-precision step): 8.22 ms per step with 0, 9.04 with 1, 8.63 with 2 -- the merged sweep
-// gathers r, v, t and p at every neighbour, which costs more than the two barriers it saves; on single
-// small domains (cylinder street, 64^2 cavity) 1 is 1-3% faster.  The workspace size depends on the choice
-// (pict_solve_workspace_bytes): switch before sizing the workspace.
+// BiCGStab kernel: 0 (default) the cluster-resident form where the cluster mode and the sizes select it, else the
+// four-barrier form on the grid; 1 the two-barrier form (NORM2 criteria, up to two right-hand sides per launch) with one
+// 512-thread CTA per SM and 128 registers per thread, 2 the same with two CTAs per SM (64 registers, some spilled); both
+// on the grid always.  Measured on the batch of 256 cavities (mixed-precision step): 8.22 ms per step with 0, 9.04 with
+// 1, 8.63 with 2 -- the merged sweep gathers r, v, t and p at every neighbour, which costs more than the two barriers it
+// saves; on single small domains (cylinder street, 64^2 cavity) 1 is 1-3% faster than the four-barrier form, which the
+// resident one halves (64^2: 161 -> 64 us a solve).  The workspace size depends on the choice (pict_solve_workspace_bytes):
+// switch before sizing the workspace.
 
 // Launch k_cg1_cluster with clusters of `cl` CTAs, as many clusters as fit on the device at once (at most
 // one per system).  Returns PICT_ERR_UNSUPPORTED (nothing launched) if no cluster of that size fits.
@@ -1980,8 +1988,11 @@ static pict_status_t launch_cg1_cluster(KArgs<T>& a, int cl, cudaStream_t st) {
 
 // ---- resident solves (krylov_resident.cuh)
 
-// Cells per thread a resident solve of this domain needs with clusters of 16 CTAs (the largest system decides;
-// every system of the domain then takes the resident path, so a batch and its members alone sum in the same order).
+// Cells per thread a resident solve of this domain needs with clusters of 16 CTAs: the largest system decides for all.
+// The sums of a resident system are ordered by its own size alone, so members of a resident batch equal their solo
+// resident solves bit for bit; the grid and k_cg1_cluster order them otherwise, so beside a ninth system or one too
+// large for the cluster a member's bits (and its iteration count by one or two) are others.  Cluster mode 0 solves every
+// batch on the grid, whose results do not depend on the other systems at all.
 static int resident_cpt(const pict_domain_t* dom) {
     const long long per_cta = ((long long)dom->max_sim_cells + KC_MAX_CL - 1) / KC_MAX_CL;
     return (int)((per_cta + RS_THREADS - 1) / RS_THREADS);
@@ -2142,7 +2153,11 @@ static pict_status_t run_solve(const pict_domain_t* dom, const void* coef, const
         a.nrhs = nrhs_total;
         void (*kern)(KArgs<T>) = nullptr;
         // few systems that fit one cluster's registers and shared memory: one launch, whose sums and waits stay in the
-        // cluster.  With many systems the lockstep grid amortises its barriers over all of them.
+        // cluster.  With many systems the lockstep grid amortises its barriers over all of them, while clusters beyond
+        // the eight or nine that run at once queue.  64^2 cavities in FP32, us a solve, grid / resident: CG 425 / 143
+        // (1 system), 479 / 270 (8), 486 / 274 (9), 480 / 400 (16), 487 / 653 (32); BiCGStab 82 / 39, 85 / 60, 90 / 62,
+        // 86 / 82, 86 / 121.  32^2 and 128^2 cross between 16 and 32 alike; the line at 8 systems is the one of
+        // k_cg1_cluster, inside the range where both win.
         const bool cg1 = !prm->use_bicg && prm->variant == 1 && a.reset == 0 && a.best == 0 && a.abs_crit == 0 && a.rankdef == 0;
         if (g_cluster_mode == 2 || (g_cluster_mode == 1 && dom->num_sims <= 8)) {
             s = PICT_ERR_UNSUPPORTED;

@@ -26,3 +26,14 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
+
+
+@pytest.fixture(params=[1, 0], ids=["clusters", "grid"])
+def krylov_mode(request):
+    """Both launch forms of the Krylov solves on a domain of few small systems: clusters (the default choice, one cluster
+    per system on chip) and the persistent grid."""
+    from pict_b200 import _lib
+    lib = _lib.load()
+    lib.pict_krylov_set_cluster_mode(request.param)
+    yield request.param
+    lib.pict_krylov_set_cluster_mode(1)

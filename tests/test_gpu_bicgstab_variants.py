@@ -1,5 +1,5 @@
-"""The two-barrier BiCGStab kernels (variants 1 and 2 of pict_krylov_set_bicgstab_variant) against the
-default four-barrier kernel (GPU):
+"""The two-barrier BiCGStab kernels (variants 1 and 2 of pict_krylov_set_bicgstab_variant) against the default
+(GPU), which is the cluster-resident kernel on these small domains and the four-barrier one on the persistent grid:
 the same iteration counts (within one) and solutions (to the solver tolerance) on single and batched
 domains, 2D and 3D, plain and transposed, FP32 and FP64, and against the oracle's BiCGStab
 (extensions/bicgstab_solver_kernel.cu:240-360)."""
@@ -33,7 +33,7 @@ def _solve(pd, b, tol, transpose, variant, conv=None):
 @pytest.mark.parametrize("transpose", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 @pytest.mark.parametrize("name", ["cavity2d", "twoblock2d_rotated", "periodic2d", "channel3d", "distorted2d"])
-def test_two_barrier_bicgstab_matches_four_barrier(name, dtype, transpose):
+def test_two_barrier_bicgstab_matches_four_barrier(name, dtype, transpose, krylov_mode):
     from pict_b200 import PISOtorch as P
     pd = build_product(case(name), dtype)
     P.SetupAdvectionMatrix(pd, torch.tensor([DT], dtype=dtype), 0)

@@ -23,7 +23,7 @@ def _relerr(a, b):
 
 @pytest.mark.parametrize("name", ALL_CASES)
 @pytest.mark.parametrize("group_size", [1, 3])
-def test_bicgstab_velocity(name, group_size):
+def test_bicgstab_velocity(name, group_size, krylov_mode):
     from pict_b200 import PISOtorch as P
     spec = case(name)
     od = build_oracle(spec)
@@ -50,7 +50,7 @@ def test_bicgstab_velocity(name, group_size):
 @pytest.mark.parametrize("name", ALL_CASES)
 @pytest.mark.parametrize("group_size", [1, 4])
 @pytest.mark.parametrize("variant", [0, 1])
-def test_cg_pressure(name, group_size, variant):
+def test_cg_pressure(name, group_size, variant, krylov_mode):
     from pict_b200 import PISOtorch as P
     spec = case(name)
     od = build_oracle(spec)
