@@ -1,7 +1,8 @@
 """Cluster CG (GPU): the single-reduction CG with one thread-block cluster per system (inner products
 through distributed shared memory, one cluster barrier per iteration) against the same recurrence on
 the persistent grid (grid-wide barriers), on batched uneven cavities, the multi-block cylinder street,
-periodic boxes and a 3D channel, FP32 and FP64, with mean removal and the blocks' pressure written.
+periodic boxes and a 3D channel, FP32 and FP64, with mean removal and the blocks' pressure written: systems small enough
+to stay on chip, and batches with one that is not (k_cg1_cluster, which keeps the vectors in memory).
 Both stop at the same RMS residual; their inner products are summed in different orders, so iteration
 counts may differ by one and solutions by the tolerance."""
 import ctypes
@@ -11,6 +12,7 @@ import pytest
 import torch
 
 from setups import build_product, case, forcing_box, lid_cavity
+from test_gpu_krylov_dispatch import _kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -27,8 +29,11 @@ def _domain(layout, dtype):
         Simulation(domain=dom, time_step=0.005, prep_fn=street_prep_fn(info), advection_tol=1e-6, pressure_tol=1e-6,
                    non_orthogonal=False).make_divergence_free()
         return dom
-    if layout == "periodic":
-        doms = [build_product(forcing_box(n), dtype) for n in (64, 40)]
+    if layout in ("periodic", "large_periodic"):
+        doms = [build_product(forcing_box(n), dtype) for n in ((64, 40) if layout == "periodic" else (272, 40))]
+        return BatchDomain(doms, time_steps=[0.01] * len(doms))
+    if layout == "large_cavities":   # 90,000 cells beside small ones
+        doms = [build_product(lid_cavity(n, viscosity=1e-3), dtype) for n in (300, 96, 64, 33)]
         return BatchDomain(doms, time_steps=[0.01] * len(doms))
     return build_product(case("channel3d"), dtype)
 
@@ -51,7 +56,7 @@ def _solve(dom, mode, rhs, tol, sub_mean):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("layout", ["cavities", "street", "periodic", "channel3d"])
+@pytest.mark.parametrize("layout", ["cavities", "street", "periodic", "channel3d", "large_cavities", "large_periodic"])
 def test_cluster_cg_matches_grid_cg(layout, dtype):
     from pict_b200.engine import PISOStepper
     dom = _domain(layout, dtype)
@@ -63,6 +68,8 @@ def test_cluster_cg_matches_grid_cg(layout, dtype):
     rms = float(rhs.double().norm()) / np.sqrt(rhs.numel())
     tol = (1e-5 if dtype == torch.float32 else 1e-11) * rms
     xg, ig, bg = _solve(dom, 0, rhs, tol, True)
+    names = _kernels(lambda: _solve(dom, 2, rhs, tol, True))
+    assert any(("k_cg1_cluster" if layout.startswith("large") else "k_cg1_resident") in m for m in names), names
     xc, ic, bc = _solve(dom, 2, rhs, tol, True)
     assert all(i.converged for i in ig) and all(i.converged for i in ic), (ig, ic)
     its_g = [i.usedIterations for i in ig]
