@@ -80,18 +80,18 @@ __device__ __forceinline__ bool mg_done(const double* sc, int sys) { return sc &
 // update kernel) applies it and skips the rest; the end-of-iteration scalar stage clears the flag.
 __device__ __forceinline__ bool mg_pending(const double* sc, int sys) { return sc && sc[MG_SC * sys + 6] != 0.0; }
 
-// First statement of every kernel of the PCG loop: wait for the previous kernel of the stream (its writes are
-// visible after the wait), then let the next one launch (programmatic dependent launch: its CTAs are
-// scheduled while this kernel's last CTAs run, and wait here in turn).  Without the launch attribute both are
-// no-ops.
+// Every kernel of the PCG loop waits for the previous kernel of the stream (its writes are visible after the wait), then
+// lets the next one launch (programmatic dependent launch: its CTAs are scheduled while this kernel's last CTAs run, and
+// wait in turn), before it reads or writes anything that a kernel of the loop writes.  Without the launch attribute
+// both are no-ops.
 __device__ __forceinline__ void mg_pdl_entry() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The parts of it, for kernels that first read what no kernel of the loop writes (tile and block tables, stencils:
-// complete before the loop's first kernel started, and a kernel's predecessor has waited for its own before this one
-// is launched), so that those reads overlap the predecessor.
+// The parts of it, for kernels that read before the wait what no kernel of the loop writes (tile and block tables,
+// stencils: complete before the loop's first kernel started, and a kernel's predecessor has waited for its own before this
+// one is launched), so that those reads overlap the predecessor.
 __device__ __forceinline__ void mg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mg_pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -635,7 +635,9 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
 // ---------------------------------------------------------------------------------------------
 // STAGED keeps the couplings in shared memory too (512 threads, two CTAs on an SM); otherwise they are read through L1
 // where they are used (256 threads, more CTAs on an SM).
-constexpr int MG2_WAVES = 4;                  // CTAs per SM up to which a launch counts as one wave
+// CTAs per SM up to which a launch counts as one wave.  PCG of N 128^2 cavities, four iterations, never / always staged:
+// 256 finest tiles 257 / 234 us, 512 291 / 285, 592 298 / 294, 768 336 / 355, 1024 377 / 404, 4096 1154 / 1243.
+constexpr int MG2_WAVES = 4;
 constexpr size_t MG2_MAX_SMEM = 192 * 1024;  // of one two-sweep CTA (FP64 stages of the widest blocks)
 constexpr int MG_TILE = 512;  // cells of a tile that the stages hold whole (the work tiles of the framework's coarse levels)
 
