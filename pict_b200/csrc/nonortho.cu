@@ -234,12 +234,11 @@ __device__ __forceinline__ T lap(const T* tr, int c1, int c2) {
 // wrapped one on a periodic axis of at least three cells, the shortest that a domain takes), so every corner is the mean
 // of its four cells: the walk around it need not be made, the own and the face neighbour's shares of the two corners of a tangential axis cancel,
 // and with them the own cell's coefficient.  What remains per pair of axes is read directly: the off-diagonal
-// coefficients of the 2 D neighbours, and for the right-hand sides the four diagonal cells.  The kernels
-// k_nonortho_plain_* take these cells and the walking kernels the others.  Measured on 96 x 65 x 80 periodic cells in
-// FP64, flags 25, walk of every cell -> plain kernel plus the walking kernel finding nothing to do: C 312 -> 66 us, P 323
-// -> 66, velocity right-hand side 1351 -> 72, pressure 438 -> 61.  The walks are bound by instructions (24 walks a cell
-// and component, each with block and face table reads); the plain kernels by L1, which serves the 19-value records of
-// the 2 D neighbours at one sector per lane.
+// coefficients of the 2 D neighbours, and for the right-hand sides the four diagonal cells.  plain_*_cells take these cells
+// and walk_*_cells the others (k_nonortho_matrix, k_nonortho_rhs).  A pass over the operators (two matrices, two right-hand
+// sides) of 96 x 65 x 80 cells in FP64, flags 25, walk of every cell -> now: periodic 2690 -> 520 us, walls in y 3290 ->
+// 690, closed 2380 -> 1650.  The walks are bound by instructions (24 walks a cell and component, each with block and
+// face table reads); the plain cells by L1, which serves the 19-value records of the 2 D neighbours at one sector per lane.
 // ---------------------------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ bool plain_cell(const pict_block_t& B, const int* p, int* off) {
@@ -269,7 +268,7 @@ __device__ __forceinline__ T plain_factor(const pict_domain_t& dom, const pict_b
 // neighbours keep a term: -+ sgn / 4 sum over the faces of the other axes of faceSign * alpha, in which the cell's own
 // half of alpha cancels between the two faces of an axis.
 template <typename T, int D, int WHICH>
-__global__ void __launch_bounds__(128) k_nonortho_plain_matrix(pict_domain_t dom, int flags, int ch) {
+__device__ __forceinline__ void plain_matrix_cells(const pict_domain_t& dom, int flags, int ch) {
     if (!(flags & NO_DIRECT_MATRIX)) return;
     const int N = dom.num_cells;
     T* M = reinterpret_cast<T*>(WHICH == 1 ? dom.P : dom.C);
@@ -306,7 +305,7 @@ __global__ void __launch_bounds__(128) k_nonortho_plain_matrix(pict_domain_t dom
 // of the lower one).  A diagonal cell is read by the two faces it is diagonal to, so its two coefficients are
 // added first: 4 values per pair of axes and component.
 template <typename T, int D, int KIND>
-__global__ void __launch_bounds__(128) k_nonortho_plain_rhs(pict_domain_t dom, int flags) {
+__device__ __forceinline__ void plain_rhs_cells(const pict_domain_t& dom, int flags) {
     constexpr int WHICH = KIND == NK_VEL ? 0 : KIND == NK_P ? 1 : 2;
     constexpr int NP = D * (D - 1) / 2;
     const int NC = KIND == NK_VEL ? D : KIND == NK_SC ? dom.scalar_channels : 1;
@@ -388,7 +387,7 @@ __global__ void __launch_bounds__(128) k_nonortho_plain_rhs(pict_domain_t dom, i
 // Neumann faces take the one-sided treatment)
 // ---------------------------------------------------------------------------------------------
 template <typename T, int D, int WHICH>
-__global__ void k_nonortho_matrix(pict_domain_t dom, int flags, int ch) {
+__device__ __forceinline__ void walk_matrix_cells(const pict_domain_t& dom, int flags, int ch) {
     constexpr int K = 2 * D + 1;
     const int N = dom.num_cells;
     T* M = reinterpret_cast<T*>(WHICH == 1 ? dom.P : dom.C);
@@ -522,7 +521,7 @@ __device__ T diagonal_data(const pict_domain_t& dom, int b, const int* p, int di
 }
 
 template <typename T, int D, int KIND>
-__global__ void k_nonortho_rhs(pict_domain_t dom, int flags) {
+__device__ __forceinline__ void walk_rhs_cells(const pict_domain_t& dom, int flags) {
     const int NC = KIND == NK_VEL ? D : KIND == NK_SC ? dom.scalar_channels : 1;
     const int N = dom.num_cells;
     const T* Ad = reinterpret_cast<const T*>(dom.A);
@@ -615,6 +614,27 @@ __global__ void k_nonortho_rhs(pict_domain_t dom, int flags) {
             else out[(size_t)c * N + i] -= S / tr_det<T, D>(tr);
         }
     }
+}
+
+// One launch an operator: the CTAs of the first row of the grid walk the cells at walls and connections, which take
+// longest and so start first, those of the second row take the plain cells at the same time.  Two launches in turn cost
+// small closed boxes more than the plain cells save.  A pass in FP32, us, walk of every cell / two launches / one: closed
+// 32^2 115 / 144 / 114, 64^2 116 / 120 / 99, 8^3 301 / 340 / 306, 16^3 348 / 371 / 338, 32^3 322 / 335 / 346, 48^3 495 / 527 /
+// 484, 64^3 987 / 830 / 680; walls in y 64^2 117 / 118 / 98, 16^3 392 / 323 / 290, 48^3 653 / 324 / 286.  Closed boxes of
+// about 40^3 are left slower than the walk of every cell (36^3 305 / 463 / 425, 40^3 371 / 494 / 448), probably because a walk
+// waits for loads there that neighbouring cells, walking too, would have brought into L1.  Not kept: lists of the walking
+// cells, walked by full warps (64^2 127, 36^3 366, 64^3 890: lanes at different walls diverge); warps that walk as a
+// whole where one cell must (36^3 308, 40^3 383, but 64^2 116, 64^3 957).
+template <typename T, int D, int WHICH>
+__global__ void __launch_bounds__(128) k_nonortho_matrix(pict_domain_t dom, int flags, int ch) {
+    if (blockIdx.y == 0) walk_matrix_cells<T, D, WHICH>(dom, flags, ch);
+    else plain_matrix_cells<T, D, WHICH>(dom, flags, ch);
+}
+
+template <typename T, int D, int KIND>
+__global__ void __launch_bounds__(128) k_nonortho_rhs(pict_domain_t dom, int flags) {
+    if (blockIdx.y == 0) walk_rhs_cells<T, D, KIND>(dom, flags);
+    else plain_rhs_cells<T, D, KIND>(dom, flags);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -936,33 +956,14 @@ static pict_status_t launch_nonortho_grad(const pict_domain_t* dom, int flags, i
 
 template <typename T, int D>
 static pict_status_t launch_nonortho(const pict_domain_t* dom, int flags, int what, int ch, cudaStream_t st) {
-    const int grid = cell_grid(dom->num_cells, 128);
-    // every cell is taken by one of the two kernels of an operator: plain_cell decides
+    const dim3 grid(cell_grid(dom->num_cells, 128), 2);
     switch (what) {
-        case 0:
-            k_nonortho_plain_matrix<T, D, 0><<<grid, 128, 0, st>>>(*dom, flags, 0);
-            k_nonortho_matrix<T, D, 0><<<grid, 128, 0, st>>>(*dom, flags, 0);
-            break;
-        case 1:
-            k_nonortho_plain_rhs<T, D, NK_VEL><<<grid, 128, 0, st>>>(*dom, flags);
-            k_nonortho_rhs<T, D, NK_VEL><<<grid, 128, 0, st>>>(*dom, flags);
-            break;
-        case 2:
-            k_nonortho_plain_matrix<T, D, 1><<<grid, 128, 0, st>>>(*dom, flags, 0);
-            k_nonortho_matrix<T, D, 1><<<grid, 128, 0, st>>>(*dom, flags, 0);
-            break;
-        case 4:
-            k_nonortho_plain_matrix<T, D, 2><<<grid, 128, 0, st>>>(*dom, flags, ch);
-            k_nonortho_matrix<T, D, 2><<<grid, 128, 0, st>>>(*dom, flags, ch);
-            break;
-        case 5:
-            k_nonortho_plain_rhs<T, D, NK_SC><<<grid, 128, 0, st>>>(*dom, flags);
-            k_nonortho_rhs<T, D, NK_SC><<<grid, 128, 0, st>>>(*dom, flags);
-            break;
-        default:
-            k_nonortho_plain_rhs<T, D, NK_P><<<grid, 128, 0, st>>>(*dom, flags);
-            k_nonortho_rhs<T, D, NK_P><<<grid, 128, 0, st>>>(*dom, flags);
-            break;
+        case 0: k_nonortho_matrix<T, D, 0><<<grid, 128, 0, st>>>(*dom, flags, 0); break;
+        case 1: k_nonortho_rhs<T, D, NK_VEL><<<grid, 128, 0, st>>>(*dom, flags); break;
+        case 2: k_nonortho_matrix<T, D, 1><<<grid, 128, 0, st>>>(*dom, flags, 0); break;
+        case 4: k_nonortho_matrix<T, D, 2><<<grid, 128, 0, st>>>(*dom, flags, ch); break;
+        case 5: k_nonortho_rhs<T, D, NK_SC><<<grid, 128, 0, st>>>(*dom, flags); break;
+        default: k_nonortho_rhs<T, D, NK_P><<<grid, 128, 0, st>>>(*dom, flags); break;
     }
     return check_launch("nonortho");
 }
