@@ -18,11 +18,13 @@
 namespace pict {
 
 // CTAs per SM that the fused assembly kernels are compiled for: six in FP32 (40 registers; 4.60 -> 4.55 ms per
-// batched step when they came from four); in FP64 that spilled 116 to 1016 bytes a thread, three leave 80 registers
-// and none (96 x 65 x 80 cells: advection matrix 75 -> 64 us, pressure matrix 48 -> 43 us).
-template <typename T>
+// batched step when they came from four).  In FP64 that spilled 116 to 1016 bytes a thread.  In 3D three leave 80
+// registers and no spills (96^3 cells, six / three: advection matrix 127 / 109 us, pressure correction 213 / 200); in 2D four
+// leave 64, whose one spill of 52 bytes costs less than fewer CTAs (1500 x 1000 cells, six / four / three: advection
+// matrix 83 / 74 / 81 us, its right-hand side 36 / 37 / 41, pressure correction 142 / 138 / 155).
+template <typename T, int D>
 struct AsmCtas {
-    static constexpr int value = sizeof(T) == 8 ? 3 : 6;
+    static constexpr int value = sizeof(T) == 8 ? (D == 3 ? 3 : 4) : 6;
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -64,7 +66,7 @@ __device__ __forceinline__ void pressure_grad_fd(const pict_domain_t& dom, const
 }
 
 template <typename T, int D, bool MATRIX, bool RHS>
-__global__ void __launch_bounds__(256, AsmCtas<T>::value) k_adv_setup(pict_domain_t dom, double dt_arg, int apply_pgrad) {
+__global__ void __launch_bounds__(256, AsmCtas<T, D>::value) k_adv_setup(pict_domain_t dom, double dt_arg, int apply_pgrad) {
     constexpr int K = 2 * D + 1;
     const int N = dom.num_cells;
     T* C = reinterpret_cast<T*>(dom.C);
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(256, AsmCtas<T>::value) k_adv_setup(pict_domai
 // ---------------------------------------------------------------------------------------------
 
 template <typename T, int D, bool MATRIX, bool RHS>
-__global__ void __launch_bounds__(256, AsmCtas<T>::value) k_pressure_setup(pict_domain_t dom, double dt_arg) {
+__global__ void __launch_bounds__(256, AsmCtas<T, D>::value) k_pressure_setup(pict_domain_t dom, double dt_arg) {
     const int N = dom.num_cells;
     const T* C = reinterpret_cast<const T*>(dom.C);
     const T* A = reinterpret_cast<const T*>(dom.A);
