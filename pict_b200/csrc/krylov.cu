@@ -219,11 +219,12 @@ __device__ void load_slots(const pict_domain_t& dom, TileSlots& S) {
     __syncthreads();
 }
 
-// Tiles of a system above which its partials are summed by the whole CTA instead of one warp.  One system, us an
-// iteration, CTA / warp: 32 tiles 6.69 / 6.62 (CG) and 24.3 / 23.6 (BiCGStab, two components), 64 tiles 6.55 / 6.77 and
-// 24.3 / 24.8, 128 tiles 6.6 / 7.5 and 24.6 / 28.2, 256 tiles 8.3 / 10.3 and 29.8 / 38.5, 1728 tiles 30 / 48 and
-// 89 / 219.  They cross at 64 tiles; up to 256 the warp's order, and so the bits of smaller systems, was kept.
-constexpr int KR_WIDE = 256;
+// Tiles of a system above which its partials are summed by the whole CTA instead of one warp.  FP32, warp / CTA, us an
+// iteration of CG and of BiCGStab with two components: one system of 118 tiles 7.1 / 6.6 and 28 / 27, of 256 9.6 / 9.4 and
+// 50 / 48, of 342 12.2 / 11.6 and 52 / 48, but eight systems, whose slots' warps sum them side by side, of 118 tiles 18 / 20
+// and 72 / 83, of 342 58 / 61 and 210 / 235.  From 1024 tiles on the CTA wins for one and for three (one: 24 / 19 and
+// 112 / 79; three: 77 / 67 and 306 / 246).
+constexpr int KR_WIDE = 512;
 
 // Sum the tile partials of each slot's system (fixed order) into out[slot][k].  Only slots whose bit is set in `mask`
 // are reduced.  A system of up to KR_WIDE tiles is summed by the slot's warp (several systems at once); a larger one by
@@ -241,7 +242,6 @@ __device__ void system_sums(const double* partials, const TileSlots& S, unsigned
         double acc[NV];
 #pragma unroll
         for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-#pragma unroll 4
         for (int t = S.t0[j] + lane; t < S.t1[j]; t += 32) {
 #pragma unroll
             for (int k = 0; k < NV; ++k) {

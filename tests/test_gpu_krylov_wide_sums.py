@@ -1,6 +1,6 @@
 """Inner products of the persistent Krylov kernels on either side of the tile count above which a whole CTA sums a
-system's partials (GPU): 256 and 257 tiles, more than one step of the CTA's threads, one tile, several of them in one
-CTA's slots.  A system's sums do not depend on the others of a batch, so a batched solve equals the solo solve bit for
+system's partials (GPU): 512 and 513 tiles, which is also one step of the CTA's threads and one more, 546, half as many,
+and one tile, several of them in one CTA's slots.  A system's sums do not depend on the others of a batch, so a batched solve equals the solo solve bit for
 bit; the residual, recomputed in FP64, is below the tolerance plus the drift of the recurrence (a few hundred roundings
 of the solution's size times the largest row sum)."""
 import ctypes
@@ -15,7 +15,7 @@ from test_gpu_resident_krylov import _box, _matrix
 pytestmark = pytest.mark.gpu
 
 TILE = 32
-SHAPES = [(192, 91), (91, 91), (257, 32), (128, 64), (6, 5)]   # 546, 259, 257, 256 and 1 tiles
+SHAPES = [(192, 91), (513, 32), (128, 128), (91, 91), (257, 32), (128, 64), (6, 5)]   # 546, 513, 512, 259, 257, 256, 1 tiles
 
 
 def _solve(shapes, rhs, tol, kind, variant, dtype):
