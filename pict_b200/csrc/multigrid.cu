@@ -629,9 +629,10 @@ __global__ void __launch_bounds__(MG_TPB, 4) k_mg_prolong(pict_mg_level_t F, pic
 // has no meaning.
 //
 // What bounds them: on few systems the latency of this chain (a level is a few CTAs), on many the shared-memory
-// reads of the sweeps over tile and halo.  Per launch of the finest level, before (256 threads, everything but b and the
-// iterates read through L1 after the wait) -> now: 16 cavities (272k cells) prolongation 10.9 -> 8.3 us, restriction
-// 16.3 -> 7.8; 256 cavities (4.34 M) prolongation 57 -> 48..55, restriction 60 -> 44..51 (69 and 57 when staged).
+// reads of the sweeps over tile and halo.  Per launch with most tiles live, launched one after the other, not staged /
+// staged: 16 cavities (272k cells) finest prolongation 10.7 / 11.5 us, finest restriction 13.9 / 9.2, the levels below 5.4 /
+// 4.2 and 7.6 / 6.2; 256 cavities (4.34 M) 97 / 119, 74 / 82, 27 / 34 and 61 / 70.  Four steps of 16 cavities 5.77 -> 4.82 ms
+// when these kernels came, of 256 cavities 24.6 -> 23.1 and now 23.0 to 23.3 with tiles of any size and masked faces.
 // ---------------------------------------------------------------------------------------------
 // STAGED keeps the couplings in shared memory too (512 threads, two CTAs on an SM); otherwise they are read through L1
 // where they are used (256 threads, more CTAs on an SM).
@@ -1676,8 +1677,7 @@ static pict_status_t run_pcg_mg(const pict_domain_t* dom, const pict_mg_level_t*
         cap_r[l] = 4 * MG_TILE + 8 * sx < MG_STAGE ? 4 * MG_TILE + 8 * sx : MG_STAGE;
         cap_p[l] = (l == 0 ? dom->tile_cells : MG_TILE) + 6 * sx;
         // the couplings too where a launch is about one wave of CTAs, whose latency counts; with several waves the
-        // kernels are bound by throughput and more CTAs on an SM hide more (256 cavities: finest prolongation 69 us
-        // staged, 48..55 not; 16 cavities: 8.3 us staged)
+        // kernels are bound by throughput and more CTAs on an SM hide more (both sides: MG2_WAVES)
         const int tr = l + 1 < nl ? levels[l + 1].num_tiles : 0, tp = l == 0 ? nt : levels[l].num_tiles;
         staged_r[l] = tr <= MG2_WAVES * device_sm_count();
         staged_p[l] = tp <= MG2_WAVES * device_sm_count();
